@@ -79,17 +79,52 @@ struct Bvh {
 };
 SST_D Bvh bvhOf(const DevScene& sc) { return Bvh{sc.nodes, sc.triv, sc.nNodes}; }
 
+// Slab offsets of a ray: a plane p lies at t = p * inv + oi when it is the near one of its axis and at
+// p * inv + of when it is the far one.  oi = of = -origin * inv, but on an axis whose direction component
+// is zero (or so small that p * inv may overflow, or NaN) these products are infinite and the slabs NaN.
+// A NaN slab is ignored by the box tests, so such a ray was culled on its other axes alone, and a lane
+// with two such axes (a cosine-distributed direction with u2 = 1 over a horizontal floor) walked most
+// of the tree while the rest of the GPU idled: on the 1M-triangle scene one path out of 67 million took
+// 300 to 800 ms of a render of 230 ms otherwise, a camera ray with one zero component 2.8 ms.
+// There inv is a power of two, so that p * inv + oi is (p - origin) * inv with one rounding: its sign
+// is exact.  The near plane is passed where it does not lie beyond the origin; the far plane is pushed
+// out by more than any distance, so that an origin exactly on it is inside as well (two triangles that
+// share an edge in the ray's plane keep it watertight).  Every box that holds a triangle such a ray can
+// meet passes, and every other ray's arithmetic is unchanged.
+SST_D void axisSlab(float o, float& inv, float& oi, float& of) {
+    oi = of = -o * inv;
+    if (!(fabsf(inv) < 1e30f)) {
+        inv = copysignf(1.2676506e30f, inv);  // 2^100
+        oi = -o * inv;
+        of = oi + fmaxf(fabsf(oi) * 1e-7f, 1e20f);
+    }
+}
+SST_D void raySlabs(float3 org, float3 dir, float3& inv, float3& oi, float3& of) {
+    inv = mk(1.0f / dir.x, 1.0f / dir.y, 1.0f / dir.z);
+    axisSlab(org.x, inv.x, oi.x, of.x);
+    axisSlab(org.y, inv.y, oi.y, of.y);
+    axisSlab(org.z, inv.z, oi.z, of.z);
+}
+// An origin that is not finite: the edge functions or the distance of every triangle are NaN, so the
+// ray misses, and its slabs could not cull anything.
+SST_D bool originLost(float3 o) { return !(fabsf(o.x) < CUDART_INF_F && fabsf(o.y) < CUDART_INF_F && fabsf(o.z) < CUDART_INF_F); }
+
+// The global id of the closest triangle so far, for a tie in t (no triangle yet loses any tie).  Read
+// back from the triangle record: ties are rare, and the register pays for the second slab offset.
+SST_D int bestId(const float4* triv, int tri) { return tri >= 0 ? __float_as_int(__ldg(&triv[3 * (size_t)tri].w)) : 0x7FFFFFFF; }
+
 // Closest hit (ANY = false; ties in t resolve to the smaller global triangle id) or any hit.
 // sstack: this block's shared stack, SSTACK entries per thread, entry k of thread `tid` at
 // k * BLOCK + tid (consecutive threads in consecutive banks).
 template <bool ANY, int BLOCK, int SSTACK>
 SST_D TraceResult traverse(const Bvh sc, float3 org, float3 dir, float tmin, float tmax, int* sstack, int* errFlags) {
     TraceResult r{tmax, 0.f, 0.f, -1};
-    if (sc.nNodes == 0 || !(tmax > tmin)) return r;
+    if (sc.nNodes == 0 || !(tmax > tmin) || originLost(org)) return r;
     int bestGid = 0x7FFFFFFF;
     RayPre pre = rayPre(dir);
-    float3 inv = mk(1.0f / dir.x, 1.0f / dir.y, 1.0f / dir.z);
-    float3 oi = mk(-org.x * inv.x, -org.y * inv.y, -org.z * inv.z);
+    float3 inv, oi, of;
+    raySlabs(org, dir, inv, oi, of);
+    const bool mx = inv.x < 0.0f, my = inv.y < 0.0f, mz = inv.z < 0.0f;  // hi is the near plane
     int lstack[kMaxStack - SSTACK];
     int sp = 0;
     uint32_t ref = 0;  // root inner node
@@ -99,18 +134,18 @@ SST_D TraceResult traverse(const Bvh sc, float3 org, float3 dir, float tmin, flo
             const float4* nd = sc.nodes + 4 * (size_t)ref;
             float4 n0 = __ldg(nd), n1 = __ldg(nd + 1), n2 = __ldg(nd + 2), n3 = __ldg(nd + 3);
             float hitT = r.t * 1.0000004f;  // conservative far bound (box/triangle rounding)
-            // child 0
-            float a0 = fmaf(n0.x, inv.x, oi.x), b0 = fmaf(n0.y, inv.x, oi.x);
-            float c0 = fmaf(n0.z, inv.y, oi.y), d0 = fmaf(n0.w, inv.y, oi.y);
-            float e0 = fmaf(n2.x, inv.z, oi.z), f0 = fmaf(n2.y, inv.z, oi.z);
-            float tn0 = fmaxf(fmaxf(fminf(a0, b0), fminf(c0, d0)), fmaxf(fminf(e0, f0), tmin));
-            float tf0 = fminf(fminf(fmaxf(a0, b0), fmaxf(c0, d0)), fminf(fmaxf(e0, f0), hitT));
+            // child 0: near and far plane of each axis
+            float a0 = fmaf(mx ? n0.y : n0.x, inv.x, oi.x), b0 = fmaf(mx ? n0.x : n0.y, inv.x, of.x);
+            float c0 = fmaf(my ? n0.w : n0.z, inv.y, oi.y), d0 = fmaf(my ? n0.z : n0.w, inv.y, of.y);
+            float e0 = fmaf(mz ? n2.y : n2.x, inv.z, oi.z), f0 = fmaf(mz ? n2.x : n2.y, inv.z, of.z);
+            float tn0 = fmaxf(fmaxf(a0, c0), fmaxf(e0, tmin));
+            float tf0 = fminf(fminf(b0, d0), fminf(f0, hitT));
             // child 1
-            float a1 = fmaf(n1.x, inv.x, oi.x), b1 = fmaf(n1.y, inv.x, oi.x);
-            float c1 = fmaf(n1.z, inv.y, oi.y), d1 = fmaf(n1.w, inv.y, oi.y);
-            float e1 = fmaf(n2.z, inv.z, oi.z), f1 = fmaf(n2.w, inv.z, oi.z);
-            float tn1 = fmaxf(fmaxf(fminf(a1, b1), fminf(c1, d1)), fmaxf(fminf(e1, f1), tmin));
-            float tf1 = fminf(fminf(fmaxf(a1, b1), fmaxf(c1, d1)), fminf(fmaxf(e1, f1), hitT));
+            float a1 = fmaf(mx ? n1.y : n1.x, inv.x, oi.x), b1 = fmaf(mx ? n1.x : n1.y, inv.x, of.x);
+            float c1 = fmaf(my ? n1.w : n1.z, inv.y, oi.y), d1 = fmaf(my ? n1.z : n1.w, inv.y, of.y);
+            float e1 = fmaf(mz ? n2.w : n2.z, inv.z, oi.z), f1 = fmaf(mz ? n2.z : n2.w, inv.z, of.z);
+            float tn1 = fmaxf(fmaxf(a1, c1), fmaxf(e1, tmin));
+            float tf1 = fminf(fminf(b1, d1), fminf(f1, hitT));
             bool h0 = tn0 <= tf0 * 1.0000004f, h1 = tn1 <= tf1 * 1.0000004f;
             uint32_t r0 = __float_as_uint(n3.x), r1 = __float_as_uint(n3.y);
             if (h0 && h1) {
@@ -182,18 +217,19 @@ SST_D float max3f(float a, float b, float c) {
     return d;
 }
 // Entry and exit distances of four child boxes from their near- and far-plane rows (x, y, z each a
-// float4 over the children): paired fused multiply-adds per plane row, then the three-operand
+// float4 over the children; oi and of the offsets of the near and of the far planes): paired fused multiply-adds per plane row, then the three-operand
 // max / min with the ray's interval.  Bitwise the scalar fmaf / fmaxf / fminf form.
-SST_D void slab4(float4 nx, float4 fx, float4 ny, float4 fy, float4 nz, float4 fz, float3 inv, float3 oi, float tmin, float tmax,
+SST_D void slab4(float4 nx, float4 fx, float4 ny, float4 fy, float4 nz, float4 fz, float3 inv, float3 oi, float3 of, float tmin, float tmax,
                  float tn[4], float tf[4]) {
     const float2 ix = make_float2(inv.x, inv.x), iy = make_float2(inv.y, inv.y), iz = make_float2(inv.z, inv.z);
     const float2 ox = make_float2(oi.x, oi.x), oy = make_float2(oi.y, oi.y), oz = make_float2(oi.z, oi.z);
+    const float2 gx = make_float2(of.x, of.x), gy = make_float2(of.y, of.y), gz = make_float2(of.z, of.z);
     const float2 nx0 = fma2(make_float2(nx.x, nx.y), ix, ox), nx1 = fma2(make_float2(nx.z, nx.w), ix, ox);
     const float2 ny0 = fma2(make_float2(ny.x, ny.y), iy, oy), ny1 = fma2(make_float2(ny.z, ny.w), iy, oy);
     const float2 nz0 = fma2(make_float2(nz.x, nz.y), iz, oz), nz1 = fma2(make_float2(nz.z, nz.w), iz, oz);
-    const float2 fx0 = fma2(make_float2(fx.x, fx.y), ix, ox), fx1 = fma2(make_float2(fx.z, fx.w), ix, ox);
-    const float2 fy0 = fma2(make_float2(fy.x, fy.y), iy, oy), fy1 = fma2(make_float2(fy.z, fy.w), iy, oy);
-    const float2 fz0 = fma2(make_float2(fz.x, fz.y), iz, oz), fz1 = fma2(make_float2(fz.z, fz.w), iz, oz);
+    const float2 fx0 = fma2(make_float2(fx.x, fx.y), ix, gx), fx1 = fma2(make_float2(fx.z, fx.w), ix, gx);
+    const float2 fy0 = fma2(make_float2(fy.x, fy.y), iy, gy), fy1 = fma2(make_float2(fy.z, fy.w), iy, gy);
+    const float2 fz0 = fma2(make_float2(fz.x, fz.y), iz, gz), fz1 = fma2(make_float2(fz.z, fz.w), iz, gz);
     tn[0] = max3f(nx0.x, ny0.x, fmaxf(nz0.x, tmin));
     tn[1] = max3f(nx0.y, ny0.y, fmaxf(nz0.y, tmin));
     tn[2] = max3f(nx1.x, ny1.x, fmaxf(nz1.x, tmin));
@@ -218,11 +254,10 @@ SST_D void cswap(float& ka, uint32_t& ra, float& kb, uint32_t& rb) {
 // hit so far stay in the structure when trav4Run pauses.
 struct Trav4 {
     Bvh4 bvh;
-    float3 org, inv, oi;
+    float3 org, inv, oi, of;
     RayPre pre;
     float tmin;
     TraceResult r;
-    int bestGid;
     int sp;
     uint32_t ref;
     uint32_t oct;  // sign bits of the inverse direction: which plane of each slab is the near one
@@ -233,15 +268,13 @@ SST_D void trav4Begin(Trav4& s, const Bvh4 bvh, float3 org, float3 dir, float tm
     s.bvh = bvh;
     s.org = org;
     s.pre = rayPre(dir);
-    s.inv = mk(1.0f / dir.x, 1.0f / dir.y, 1.0f / dir.z);
-    s.oi = mk(-org.x * s.inv.x, -org.y * s.inv.y, -org.z * s.inv.z);
+    raySlabs(org, dir, s.inv, s.oi, s.of);
     s.oct = (s.inv.x < 0.0f ? 1u : 0u) | (s.inv.y < 0.0f ? 2u : 0u) | (s.inv.z < 0.0f ? 4u : 0u);
     s.tmin = tmin;
     s.r = TraceResult{tmax, 0.f, 0.f, -1};
-    s.bestGid = 0x7FFFFFFF;
     s.sp = 0;
     s.ref = 0;  // root
-    s.done = bvh.nNodes4 == 0 || !(tmax > tmin);
+    s.done = bvh.nNodes4 == 0 || !(tmax > tmin) || originLost(org);
 }
 
 // Traversal steps until the ray is finished (returns true, result in s.r) or, with pauseIdle > 0,
@@ -264,8 +297,7 @@ SST_D bool trav4Run(Trav4& s, int* sstack, int* lstack, int* errFlags, int pause
             // the near plane of each slab is lo for a positive direction component and hi for a
             // negative one; its t is then the smaller of the two (fma rounding is monotonic), so
             // reading the near and far planes directly gives the min / max of both without computing
-            // them.  With an infinite inverse (a zero component) a NaN slab is ignored, which keeps
-            // at least the boxes the min / max form keeps.
+            // them.
             const int ox = (int)(s.oct & 1u), oy = (int)((s.oct >> 1) & 1u), oz = (int)((s.oct >> 2) & 1u);
             const float4 nx = __ldg(nd + ox), fx = __ldg(nd + 1 - ox), ny = __ldg(nd + 2 + oy), fy = __ldg(nd + 3 - oy);
             const float4 nz = __ldg(nd + 4 + oz), fz = __ldg(nd + 5 - oz);
@@ -276,7 +308,7 @@ SST_D bool trav4Run(Trav4& s, int* sstack, int* lstack, int* errFlags, int pause
             uint32_t cr[4];
             const float* RF = &rf.x;
             float tn[4], tf[4];
-            slab4(nx, fx, ny, fy, nz, fz, s.inv, s.oi, s.tmin, hitT, tn, tf);
+            slab4(nx, fx, ny, fy, nz, fz, s.inv, s.oi, s.of, s.tmin, hitT, tn, tf);
             int nh = 0;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
@@ -315,7 +347,7 @@ SST_D bool trav4Run(Trav4& s, int* sstack, int* lstack, int* errFlags, int pause
                 if (isectTri(s.org, s.pre, f3(a), f3(b), f3(c), s.tmin, lim, t, u, v)) {
                     int gid = __float_as_int(a.w);
                     if (ANY) { s.r.t = t; s.r.u = u; s.r.v = v; s.r.tri = ti; return true; }
-                    if (t < s.r.t || (t == s.r.t && gid < s.bestGid)) { s.r.t = t; s.r.u = u; s.r.v = v; s.r.tri = ti; s.bestGid = gid; }
+                    if (t < s.r.t || (t == s.r.t && gid < bestId(sc.triv, s.r.tri))) { s.r.t = t; s.r.u = u; s.r.v = v; s.r.tri = ti; }
                 }
             }
         }
@@ -329,11 +361,8 @@ SST_D bool trav4Run(Trav4& s, int* sstack, int* lstack, int* errFlags, int pause
 // node's hit children in the order slot ^ o ascending, o the sign bits of its direction, which
 // approximates front to back without a sort.  A node visit tests the eight child boxes against the
 // near and far planes the direction selects (the near-plane arrays are read directly, so every
-// slab is one fused multiply-add).  It is the other widths' arithmetic: with a finite inverse
-// direction the near plane's t is the smaller of the two, so a box passes here exactly when it
-// passes there, and with an infinite one (a zero direction component) a NaN slab is ignored, which
-// passes at least the boxes the other widths pass.  The hit children become a bit mask in visiting
-// order.  The
+// slab is one fused multiply-add).  It is the other widths' arithmetic, so a box passes here exactly
+// when it passes there.  The hit children become a bit mask in visiting order.  The
 // traversal keeps one (node, remaining mask) group in registers; moving to an inner child pushes
 // the rest of the group as one stack entry (node << 8 | mask), and a leaf child is tested in
 // place.  SSTACK entries per thread in shared memory, the rest in local memory (the depth of the
@@ -347,11 +376,10 @@ SST_D Bvh8 bvh8Of(const DevScene& sc) { return Bvh8{sc.nodes8, sc.triv, sc.nNode
 
 struct Trav8 {
     Bvh8 bvh;
-    float3 org, inv, oi;
+    float3 org, inv, oi, of;
     RayPre pre;
     float tmin;
     TraceResult r;
-    int bestGid;
     int sp;
     uint32_t node;  // the group in registers: an 8-wide node ...
     uint32_t mask;  // ... and its hit children not yet visited (bit j: slot j ^ oct)
@@ -374,7 +402,7 @@ SST_D uint32_t visit8(const Trav8& s, uint32_t node) {
         const float4 ny = __ldg(nd + 4 + 2 * oy + h), fy = __ldg(nd + 6 - 2 * oy + h);
         const float4 nz = __ldg(nd + 8 + 2 * oz + h), fz = __ldg(nd + 10 - 2 * oz + h);
         float tn[4], tf[4];
-        slab4(nx, fx, ny, fy, nz, fz, s.inv, s.oi, s.tmin, hitT, tn, tf);
+        slab4(nx, fx, ny, fy, nz, fz, s.inv, s.oi, s.of, s.tmin, hitT, tn, tf);
 #pragma unroll
         for (int k = 0; k < 4; ++k) hm |= (tn[k] <= tf[k] * 1.0000004f) ? (1u << (4 * h + k)) : 0u;
     }
@@ -390,15 +418,13 @@ SST_D void trav8Begin(Trav8& s, const Bvh8 bvh, float3 org, float3 dir, float tm
     s.bvh = bvh;
     s.org = org;
     s.pre = rayPre(dir);
-    s.inv = mk(1.0f / dir.x, 1.0f / dir.y, 1.0f / dir.z);
-    s.oi = mk(-org.x * s.inv.x, -org.y * s.inv.y, -org.z * s.inv.z);
+    raySlabs(org, dir, s.inv, s.oi, s.of);
     s.oct = (s.inv.x < 0.0f ? 1u : 0u) | (s.inv.y < 0.0f ? 2u : 0u) | (s.inv.z < 0.0f ? 4u : 0u);
     s.tmin = tmin;
     s.r = TraceResult{tmax, 0.f, 0.f, -1};
-    s.bestGid = 0x7FFFFFFF;
     s.sp = 0;
     s.node = 0;
-    s.done = bvh.nNodes8 == 0 || !(tmax > tmin);
+    s.done = bvh.nNodes8 == 0 || !(tmax > tmin) || originLost(org);
     s.mask = s.done ? 0u : visit8(s, 0u);  // the root's hit children
     if (!s.done && s.mask == 0u) s.done = true;
 }
@@ -446,7 +472,7 @@ SST_D bool trav8Run(Trav8& s, int* sstack, int* lstack, int* errFlags, int pause
                 if (isectTri(s.org, s.pre, f3(a), f3(b), f3(c), s.tmin, lim, t, u, v)) {
                     const int gid = __float_as_int(a.w);
                     if (ANY) { s.r.t = t; s.r.u = u; s.r.v = v; s.r.tri = ti; return true; }
-                    if (t < s.r.t || (t == s.r.t && gid < s.bestGid)) { s.r.t = t; s.r.u = u; s.r.v = v; s.r.tri = ti; s.bestGid = gid; }
+                    if (t < s.r.t || (t == s.r.t && gid < bestId(s.bvh.triv, s.r.tri))) { s.r.t = t; s.r.u = u; s.r.v = v; s.r.tri = ti; }
                 }
             }
         }
