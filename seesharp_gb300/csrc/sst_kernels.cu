@@ -397,8 +397,63 @@ void launch_film_fold(const DevJob* jobs, const WaveChunk* chunks, const WaveDes
 // queue order the expensive surface shading runs in every warp with the cheap lanes idle beside
 // it; ordered, it runs in fewer, fuller warps.  Every path's result is the same in any order.
 // counts[0], counts[1]: this bounce's append counters (zeroed with the wave's counters).
-__global__ void __launch_bounds__(256) k_partition(const uint32_t* __restrict__ depth, const float4* __restrict__ hits, const int* nIn, int* order,
-                                                    int* counts) {
+// A block orders kPartItems paths with one addition to each counter.  With one per warp the launch was
+// bound by those two addresses: 28.2 us for 2^20 paths of the Cornell box (65536 additions, DRAM at 9%
+// of peak) against 13.1 us.
+constexpr int kPartThreads = 256, kPartPer = 4, kPartItems = kPartThreads * kPartPer;
+__global__ void __launch_bounds__(kPartThreads) k_partition(const uint32_t* __restrict__ depth, const float4* __restrict__ hits, const int* nIn,
+                                                             int* order, int* counts) {
+    constexpr int kSlices = kPartItems / 32;  // the warps of the block, kPartPer times
+    static_assert(kSlices == 32, "one lane per slice in the scan below");
+    __shared__ int before[2][kSlices];
+    const int n = *nIn;
+    const int first = blockIdx.x * kPartItems;
+    if (first >= n) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    unsigned ms[kPartPer], mo[kPartPer];
+#pragma unroll
+    for (int k = 0; k < kPartPer; ++k) {
+        const int i = first + k * kPartThreads + (int)threadIdx.x;
+        const bool valid = i < n;
+        const bool surf = valid && !(depth[i] & kDoneFlag) && __float_as_int(hits[i].w) >= 0;
+        ms[k] = __ballot_sync(0xffffffffu, surf);
+        mo[k] = __ballot_sync(0xffffffffu, valid && !surf);
+        if (lane == 0) {
+            before[0][k * (kPartThreads / 32) + warp] = __popc(ms[k]);
+            before[1][k * (kPartThreads / 32) + warp] = __popc(mo[k]);
+        }
+    }
+    __syncthreads();
+    if (warp < 2) {  // warp 0: the surface hits, warp 1: the others
+        const int c = before[warp][lane];
+        int sum = c;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += v;
+        }
+        int base = 0;
+        if (lane == 31 && sum > 0) base = atomicAdd(&counts[warp], sum);
+        base = __shfl_sync(0xffffffffu, base, 31);
+        before[warp][lane] = base + sum - c;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kPartPer; ++k) {
+        const int i = first + k * kPartThreads + (int)threadIdx.x, slice = k * (kPartThreads / 32) + warp;
+        if (ms[k] >> lane & 1u) order[before[0][slice] + __popc(ms[k] & below)] = i;                    // from the front
+        else if (mo[k] >> lane & 1u) order[n - 1 - (before[1][slice] + __popc(mo[k] & below))] = i;   // from the back
+    }
+}
+
+// The same with one addition per warp, for the adjoint replay: its gradients are sums of millions of
+// 32-bit additions of warp sums, whose rounding depends on which paths share a warp.  With the order
+// above the emitter gradients of the differentiable Cornell box (512^2, 32 spp) moved by a relative
+// 3e-4, 20 times what they vary by from run to run, so the replay keeps the order they always had.
+// Also for waves of up to 2^16 paths, whose at most 2 x 2048 additions are no bound and whose few blocks
+// of the kernel above would take longer than many small ones (160 x 90 preview: 2% faster with this).
+__global__ void __launch_bounds__(256) k_partition_warp(const uint32_t* __restrict__ depth, const float4* __restrict__ hits, const int* nIn, int* order,
+                                                         int* counts) {
     const int n = *nIn;
     if ((int)(blockIdx.x * blockDim.x) >= n) return;  // whole blocks: every warp below is complete
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -418,10 +473,14 @@ __global__ void __launch_bounds__(256) k_partition(const uint32_t* __restrict__ 
     else if (valid) order[n - 1 - (bo + __popc(mo & below))] = i;   // from the back
 }
 
-void launch_partition(const uint32_t* depth, const float4* hits, const int* nIn, int* order, int* counts, int maxItems, cudaStream_t s) {
-    const int grid = (maxItems + 255) / 256;
+void launch_partition(bool replay, const uint32_t* depth, const float4* hits, const int* nIn, int* order, int* counts, int maxItems, cudaStream_t s) {
+    if (replay || maxItems <= (1 << 16)) {
+        if (maxItems > 0) k_partition_warp<<<(maxItems + 255) / 256, 256, 0, s>>>(depth, hits, nIn, order, counts);
+        return;
+    }
+    const int grid = (maxItems + kPartItems - 1) / kPartItems;
     if (grid == 0) return;
-    k_partition<<<grid, 256, 0, s>>>(depth, hits, nIn, order, counts);
+    k_partition<<<grid, kPartThreads, 0, s>>>(depth, hits, nIn, order, counts);
 }
 
 bool shadeBlocksValid(int b) { return b == SST_SHADE_GEN_MIN_BLOCKS || b == 10 || b == 12 || b == SST_SHADE_GEN_DENSE_BLOCKS; }

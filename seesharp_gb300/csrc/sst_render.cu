@@ -296,7 +296,7 @@ void renderJobs(sst_ctx* c, std::vector<JobIn>& jobs, SstRenderStats* out, bool 
                 PathBuf Ao = A;
                 if (split) Ao.rec = sk.rec.as<float4>();
                 if (c->shadeOrder) {
-                    launch_partition(A.depth, wb.hits, cnt + kCntQueue + d, wb.order, cnt + kCntPart + 2 * d, maxItems, rs);
+                    launch_partition(replay, A.depth, wb.hits, cnt + kCntQueue + d, wb.order, cnt + kCntPart + 2 * d, maxItems, rs);
                     Ao.order = wb.order;
                 }
                 // next-event slots: read the buffer the previous bounce wrote, write the other
