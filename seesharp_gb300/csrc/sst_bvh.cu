@@ -13,6 +13,8 @@
 //      child boxes in the parent, 64-byte nodes); a collapsed subtree becomes one leaf reference
 //      to its contiguous range of sorted triangles.
 #include <cub/cub.cuh>
+#include <thrust/iterator/counting_iterator.h>
+#include <thrust/iterator/transform_iterator.h>
 #include <math_constants.h>
 #include <algorithm>
 #include <cstdlib>
@@ -29,6 +31,12 @@ namespace {
 // 1M-triangle scene it traverses 3.4% faster than 1.0 (and 1.0 17% faster than 3.0).
 constexpr float kCt = 0.25f;
 constexpr float kCi = 1.0f;
+// PLOC rounds between two looks at the cluster count.  A round leaves 70 to 80% of the clusters, so the
+// third one's grid is at most twice what it needs.  With a look (four read-backs and a wait) after every
+// one of the 61 rounds of 614K triangles the GPU idled for half of a commit: 8.8 ms against 5.1 ms with a
+// look after every third round and one block for the last half of them (and the wide tree's levels
+// launched from bounds); 36 triangles: 1.11 against 0.27 ms.
+constexpr int kPlocRounds = 3;
 
 __device__ __forceinline__ int floatOrd(float f) {
     int i = __float_as_int(f);
@@ -222,58 +230,184 @@ __global__ void k_ploc_init(const float4* tri, const int* order, int n, int* clu
     clus[i] = ~i;
 }
 
-// nearest neighbour within `radius` positions (ties: the smaller index)
-__global__ void k_ploc_nn(const float* cbox, const int* nc, int radius, int* nn) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int n = *nc;
+// Nearest neighbour within `radius` positions (ties: the smaller index).  A block keeps its clusters'
+// boxes and those of `radius` positions on both sides in shared memory (every box is read up to
+// 2 radius + 1 times).  Blocks past the *nc clusters have nothing to do.
+constexpr int kNnThreads = 256;
+constexpr int kPlocMaxRadius = 256;
+__global__ void __launch_bounds__(kNnThreads) k_ploc_nn(const float* cbox, const int* nc, int radius, int* nn) {
+    __shared__ float box[6][kNnThreads + 2 * kPlocMaxRadius];
+    const int n = *nc, first = blockIdx.x * kNnThreads;
+    if (first >= n) return;
+    const int lo = max(0, first - radius), hi = min(n, first + kNnThreads + radius);
+    for (int e = threadIdx.x; e < 6 * (hi - lo); e += kNnThreads) box[e % 6][e / 6] = cbox[6 * (size_t)lo + e];
+    __syncthreads();
+    const int i = first + threadIdx.x;
     if (i >= n) return;
     float me[6];
-    for (int k = 0; k < 6; ++k) me[k] = cbox[6 * (size_t)i + k];
+    for (int k = 0; k < 6; ++k) me[k] = box[k][i - lo];
     float best = CUDART_INF_F;
     int bj = -1;
-    int j0 = max(0, i - radius), j1 = min(n - 1, i + radius);
+    const int j0 = max(0, i - radius), j1 = min(n - 1, i + radius);
     for (int j = j0; j <= j1; ++j) {
         if (j == i) continue;
-        float a = unionArea(me, cbox + 6 * (size_t)j);
+        const float o[6] = {box[0][j - lo], box[1][j - lo], box[2][j - lo], box[3][j - lo], box[4][j - lo], box[5][j - lo]};
+        float a = unionArea(me, o);
         if (a < best) { best = a; bj = j; }
     }
     nn[i] = bj;
 }
 
-// flags: create[i] = i merges with its mutual neighbour (i the lower index); keep[i] = cluster i
-// (possibly merged) stays in the list
-__global__ void k_ploc_flags(const int* nn, const int* nc, int* create, int* keep) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int n = *nc;
-    if (i >= n) return;
-    int j = nn[i];
-    bool mutual = j >= 0 && nn[j] == i;
-    create[i] = (mutual && i < j) ? 1 : 0;
-    keep[i] = (!mutual || i < j) ? 1 : 0;
-}
+// What becomes of cluster i, as one 64-bit item for a single scan of both: bit 0: it stays in the list
+// (possibly merged), bit 32: it merges with its mutual nearest neighbour (it is the lower of the two).
+// Items past the *nc clusters are zero, so that a scan over a larger count gives the same sums.
+struct PlocFlags {
+    const int* nn;
+    const int* nc;
+    __device__ __forceinline__ unsigned long long operator()(int i) const {
+        if (i >= *nc) return 0ull;
+        const int j = nn[i];
+        const bool mutual = j >= 0 && nn[j] == i;
+        return ((mutual && i < j) ? (1ull << 32) : 0ull) | ((!mutual || i < j) ? 1ull : 0ull);
+    }
+};
 
-// merged clusters become inner nodes numbered base + createIdx[i] in creation order
-__global__ void k_ploc_compact(const int* clus, const float* cbox, const int* nn, const int* nc, const int* create, const int* createIdx,
-                               const int* keep, const int* newPos, int base, int* clusOut, float* cboxOut, int2* child, float* ibox) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int n = *nc;
-    if (i >= n || !keep[i]) return;
-    int out = newPos[i];
-    if (create[i]) {
-        int j = nn[i];
-        int id = base + createIdx[i];
+// Merged clusters become inner nodes in creation order: so far n - *nc of them, since every merge leaves
+// one cluster less.  The last cluster's thread writes the new count.
+__global__ void k_ploc_compact(const int* clus, const float* cbox, const int* nn, const int* nc, int n, const unsigned long long* before, int* clusOut,
+                               float* cboxOut, int* ncOut, int2* child) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int m = *nc;
+    if (i >= m) return;
+    const unsigned long long f = PlocFlags{nn, nc}(i), at = before[i];
+    const int out = (int)(uint32_t)at;
+    if (i == m - 1) *ncOut = out + (int)(f & 1u);
+    if (!(f & 1u)) return;
+    float b[6];
+    for (int k = 0; k < 6; ++k) b[k] = cbox[6 * (size_t)i + k];
+    if (f >> 32) {
+        const int j = nn[i], id = n - m + (int)(at >> 32);
         child[id] = make_int2(clus[i], clus[j]);
-        float* b = cboxOut + 6 * (size_t)out;
         for (int k = 0; k < 3; ++k) {
-            b[k] = fminf(cbox[6 * (size_t)i + k], cbox[6 * (size_t)j + k]);
-            b[3 + k] = fmaxf(cbox[6 * (size_t)i + 3 + k], cbox[6 * (size_t)j + 3 + k]);
+            b[k] = fminf(b[k], cbox[6 * (size_t)j + k]);
+            b[3 + k] = fmaxf(b[3 + k], cbox[6 * (size_t)j + 3 + k]);
         }
-        for (int k = 0; k < 6; ++k) ibox[6 * (size_t)id + k] = b[k];
         clusOut[out] = id;
     } else {
         clusOut[out] = clus[i];
-        for (int k = 0; k < 6; ++k) cboxOut[6 * (size_t)out + k] = cbox[6 * (size_t)i + k];
     }
+    for (int k = 0; k < 6; ++k) cboxOut[6 * (size_t)out + k] = b[k];
+}
+
+// The remaining rounds of at most kTailClusters clusters in one block, boxes and references in shared
+// memory: the same searches, merges and numbering.  About half of all rounds run on so few clusters, and
+// as separate launches each costs tens of microseconds of launches and a wait for a few thousand items.
+// Leaves the cluster count in *nc: 1 when the tree is complete, more when no pair merges (NaN boxes).
+constexpr int kTailThreads = 1024, kTailPer = 4, kTailClusters = kTailThreads * kTailPer;
+constexpr int kTailSlices = kTailClusters / 32;
+constexpr size_t kTailSmem = sizeof(float) * 6 * kTailClusters + sizeof(int) * 2 * kTailClusters;
+__global__ void __launch_bounds__(kTailThreads) k_ploc_tail(const int* clusIn, const float* cboxIn, int* nc, int n, int radius, int2* child) {
+    extern __shared__ float tailMem[];
+    float* const box = tailMem;                                              // [6][kTailClusters]
+    int* const clus = reinterpret_cast<int*>(box + 6 * kTailClusters);
+    int* const nn = clus + kTailClusters;
+    __shared__ int2 before[kTailSlices];  // (kept, created) in the slices of 32 clusters before
+    __shared__ int2 total;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    int m = *nc;
+    if (m > kTailClusters) return;
+    for (int e = tid; e < 6 * m; e += kTailThreads) box[(e % 6) * kTailClusters + e / 6] = cboxIn[e];
+    for (int i = tid; i < m; i += kTailThreads) clus[i] = clusIn[i];
+    __syncthreads();
+    while (m > 1) {
+        for (int i = tid; i < m; i += kTailThreads) {
+            float me[6];
+            for (int k = 0; k < 6; ++k) me[k] = box[k * kTailClusters + i];
+            float best = CUDART_INF_F;
+            int bj = -1;
+            const int j0 = max(0, i - radius), j1 = min(m - 1, i + radius);
+            for (int j = j0; j <= j1; ++j) {
+                if (j == i) continue;
+                float o[6];
+                for (int k = 0; k < 6; ++k) o[k] = box[k * kTailClusters + j];
+                const float a = unionArea(me, o);
+                if (a < best) { best = a; bj = j; }
+            }
+            nn[i] = bj;
+        }
+        __syncthreads();
+        unsigned keep[kTailPer], make[kTailPer];
+        int ref[kTailPer];
+        float nb[kTailPer][6];
+        int2 pair[kTailPer];
+#pragma unroll
+        for (int q = 0; q < kTailPer; ++q) {
+            const int i = q * kTailThreads + tid;
+            bool kp = false, mk = false;
+            if (i < m) {
+                const int j = nn[i];
+                const bool mutual = j >= 0 && nn[j] == i;
+                mk = mutual && i < j;
+                kp = !mutual || i < j;
+                if (kp) {
+                    for (int k = 0; k < 6; ++k) nb[q][k] = box[k * kTailClusters + i];
+                    ref[q] = clus[i];
+                    if (mk) {
+                        for (int k = 0; k < 3; ++k) {
+                            nb[q][k] = fminf(nb[q][k], box[k * kTailClusters + j]);
+                            nb[q][3 + k] = fmaxf(nb[q][3 + k], box[(3 + k) * kTailClusters + j]);
+                        }
+                        pair[q] = make_int2(ref[q], clus[j]);
+                    }
+                }
+            }
+            keep[q] = __ballot_sync(0xffffffffu, kp);
+            make[q] = __ballot_sync(0xffffffffu, mk);
+            if (lane == 0) before[q * (kTailThreads / 32) + warp] = make_int2(__popc(keep[q]), __popc(make[q]));
+        }
+        __syncthreads();
+        if (warp == 0) {
+            constexpr int per = kTailSlices / 32;
+            int2 own[per], sum = make_int2(0, 0);
+            for (int k = 0; k < per; ++k) {
+                own[k] = before[lane * per + k];
+                sum.x += own[k].x;
+                sum.y += own[k].y;
+            }
+            int2 inc = sum;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int x = __shfl_up_sync(0xffffffffu, inc.x, o), y = __shfl_up_sync(0xffffffffu, inc.y, o);
+                if (lane >= o) { inc.x += x; inc.y += y; }
+            }
+            int2 at = make_int2(inc.x - sum.x, inc.y - sum.y);
+            for (int k = 0; k < per; ++k) {
+                before[lane * per + k] = at;
+                at.x += own[k].x;
+                at.y += own[k].y;
+            }
+            if (lane == 31) total = inc;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < kTailPer; ++q) {
+            if (!(keep[q] >> lane & 1u)) continue;
+            const int2 at = before[q * (kTailThreads / 32) + warp];
+            const int out = at.x + __popc(keep[q] & below);
+            if (make[q] >> lane & 1u) {
+                const int id = n - m + at.y + __popc(make[q] & below);
+                child[id] = pair[q];
+                ref[q] = id;
+            }
+            clus[out] = ref[q];
+            for (int k = 0; k < 6; ++k) box[k * kTailClusters + out] = nb[q][k];
+        }
+        const int2 t = total;
+        __syncthreads();
+        m = t.x;
+        if (t.y == 0) break;  // no mutual pair: boxes that are not numbers
+    }
+    if (tid == 0) *nc = m;
 }
 
 // creation ids -> final ids (root = 0: reversed creation order); parent pointers
@@ -413,7 +547,10 @@ static size_t cubTempBytes(int n) {
     cub::DeviceRadixSort::SortPairs(nullptr, sortBytes, (unsigned long long*)nullptr, (unsigned long long*)nullptr, (int*)nullptr, (int*)nullptr, n,
                                     0, 63);
     cub::DeviceScan::ExclusiveSum(nullptr, scanBytes, (int*)nullptr, (int*)nullptr, n > 1 ? n - 1 : 1);
-    return std::max(sortBytes, scanBytes);
+    size_t plocBytes = 0;
+    cub::DeviceScan::ExclusiveSum(nullptr, plocBytes, thrust::make_transform_iterator(thrust::make_counting_iterator<int>(0), PlocFlags{nullptr, nullptr}),
+                                  (unsigned long long*)nullptr, n);
+    return std::max(std::max(sortBytes, scanBytes), plocBytes);
 }
 
 size_t lbvhScratchBytes(int n) {
@@ -424,7 +561,7 @@ size_t lbvhScratchBytes(int n) {
     s += sizeof(int) * n * 2;                                        // parents
     s += sizeof(int) * n * 4;                                        // visits, collapse, kept, newIdx
     s += sizeof(float) * n * 7;                                      // boxes, cost
-    s += sizeof(int) * n * 11 + sizeof(float) * n * 18 + sizeof(int2) * n + 4096;  // PLOC clusters, boxes, flags, sizes
+    s += sizeof(int) * n * 6 + sizeof(unsigned long long) * n + sizeof(float) * n * 12 + sizeof(int2) * n + 4096;  // PLOC clusters, positions, boxes, sizes
     s += tmp + 64 * 256 + 64;
     return s;
 }
@@ -477,12 +614,8 @@ int buildLbvh(const float4* tri, int n, float4* nodesOut, int* orderOut, void* s
         int* clus2 = carve<int>(p, n);
         float* cbox = carve<float>(p, 6 * size_t(n));
         float* cbox2 = carve<float>(p, 6 * size_t(n));
-        float* ibox = carve<float>(p, 6 * size_t(n));
         int* nn = carve<int>(p, n);
-        int* create = carve<int>(p, n);
-        int* keep = carve<int>(p, n);
-        int* createIdx = carve<int>(p, n);
-        int* newPos = carve<int>(p, n);
+        unsigned long long* before = carve<unsigned long long>(p, n);
         int* nc = carve<int>(p, 4);
         int2* childC = carve<int2>(p, n);
         int* size = carve<int>(p, n);
@@ -490,33 +623,34 @@ int buildLbvh(const float4* tri, int n, float4* nodesOut, int* orderOut, void* s
         int* order2 = carve<int>(p, n);
         if (size_t(p - static_cast<char*>(scratch)) > scratchBytes) return -2;
         k_ploc_init<<<grid, 256, 0, st>>>(tri, valsB, n, clus, cbox);
-        int ncH = n, base = 0;
+        // Every round reads the cluster count on the device; the host's figure only bounds the grids and
+        // the scan, so it is read back once every few rounds, until one block can do the rest.
+        int ncH = n, cur = 0;
         cudaMemcpyAsync(nc, &ncH, sizeof(int), cudaMemcpyHostToDevice, st);
-        size_t scanBytes = 0;
-        cub::DeviceScan::ExclusiveSum(nullptr, scanBytes, create, createIdx, n, st);
-        if (scanBytes > tmpBytes) return -2;
-        for (int round = 0; ncH > 1; ++round) {
-            if (round > n) return -3;  // each round merges at least the globally closest pair
-            int g = (ncH + 255) / 256;
-            k_ploc_nn<<<g, 256, 0, st>>>(cbox, nc, plocRadius, nn);
-            k_ploc_flags<<<g, 256, 0, st>>>(nn, nc, create, keep);
-            cub::DeviceScan::ExclusiveSum(tmp, scanBytes, create, createIdx, ncH, st);
-            cub::DeviceScan::ExclusiveSum(tmp, scanBytes, keep, newPos, ncH, st);
-            k_ploc_compact<<<g, 256, 0, st>>>(clus, cbox, nn, nc, create, createIdx, keep, newPos, base, clus2, cbox2, childC, ibox);
-            int h4[4];
-            cudaMemcpyAsync(&h4[0], createIdx + (ncH - 1), sizeof(int), cudaMemcpyDeviceToHost, st);
-            cudaMemcpyAsync(&h4[1], create + (ncH - 1), sizeof(int), cudaMemcpyDeviceToHost, st);
-            cudaMemcpyAsync(&h4[2], newPos + (ncH - 1), sizeof(int), cudaMemcpyDeviceToHost, st);
-            cudaMemcpyAsync(&h4[3], keep + (ncH - 1), sizeof(int), cudaMemcpyDeviceToHost, st);
+        static_assert(kTailSmem <= 200 * 1024, "shared memory of the tail block");
+        if (cudaFuncSetAttribute(k_ploc_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTailSmem)) != cudaSuccess) return -1;
+        while (ncH > kTailClusters) {
+            for (int r = 0; r < kPlocRounds; ++r) {
+                const int* ncIn = nc + cur;
+                k_ploc_nn<<<(ncH + kNnThreads - 1) / kNnThreads, kNnThreads, 0, st>>>(cbox, ncIn, plocRadius, nn);
+                auto flags = thrust::make_transform_iterator(thrust::make_counting_iterator<int>(0), PlocFlags{nn, ncIn});
+                size_t scanBytes = tmpBytes;
+                if (cub::DeviceScan::ExclusiveSum(tmp, scanBytes, flags, before, ncH, st) != cudaSuccess) return -2;
+                k_ploc_compact<<<(ncH + 255) / 256, 256, 0, st>>>(clus, cbox, nn, ncIn, n, before, clus2, cbox2, nc + (1 - cur), childC);
+                cur = 1 - cur;
+                std::swap(clus, clus2);
+                std::swap(cbox, cbox2);
+            }
+            int left = 0;
+            cudaMemcpyAsync(&left, nc + cur, sizeof(int), cudaMemcpyDeviceToHost, st);
             if (cudaStreamSynchronize(st) != cudaSuccess) return -1;
-            if (h4[0] + h4[1] == 0) return -3;  // no mutual pair: degenerate boxes
-            base += h4[0] + h4[1];
-            ncH = h4[2] + h4[3];
-            cudaMemcpyAsync(nc, &ncH, sizeof(int), cudaMemcpyHostToDevice, st);
-            std::swap(clus, clus2);
-            std::swap(cbox, cbox2);
+            if (left >= ncH || left < 1) return -3;  // every round merges at least the closest pair: degenerate boxes
+            ncH = left;
         }
-        if (base != n - 1) return -4;
+        k_ploc_tail<<<1, kTailThreads, kTailSmem, st>>>(clus, cbox, nc + cur, n, plocRadius, childC);
+        cudaMemcpyAsync(&ncH, nc + cur, sizeof(int), cudaMemcpyDeviceToHost, st);
+        if (cudaStreamSynchronize(st) != cudaSuccess) return -1;
+        if (ncH != 1) return -3;
         k_ploc_renumber<<<grid, 256, 0, st>>>(childC, n, child, parentInner, parentLeaf);
         cudaMemsetAsync(size, 0, sizeof(int) * n, st);
         k_ploc_sizes<<<grid, 256, 0, st>>>(child, parentLeaf, parentInner, n, visits, size);
@@ -586,7 +720,7 @@ void launch_leaf_gather(const int* order, int n, const float4* trivG, const floa
 // 4-wide BVH from the binary one.  Each 4-wide node is made from a binary inner node by opening
 // its inner children with the largest surface area until it has four children (or only leaves
 // remain); leaves are shared unchanged.  Level-synchronous: one launch per level of the 4-wide
-// tree, the frontier holds (binary node, 4-wide slot) pairs.
+// tree, the frontier holds the level's binary nodes in the order of their 4-wide slots.
 // Node layout (8 float4, 128 bytes): lo.x[4], hi.x[4], lo.y[4], hi.y[4], lo.z[4], hi.z[4],
 // child references[4] (a 4-wide node index or a leaf reference), (number of children, -, -, -).
 // =============================================================================================
@@ -608,14 +742,46 @@ __device__ void readChildren(const float4* nodes2, uint32_t b, Child4& c0, Child
     c0.ref = __float_as_uint(n3.x);
     c1.ref = __float_as_uint(n3.y);
 }
-__global__ void k_collapse4(const float4* nodes2, const int2* frontier, const int* nFront, float4* nodes4, int* nodeCounter, int2* next,
-                            int* nNext) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= *nFront) return;
-    int2 item = frontier[i];
+// The levels of a wide build: the number of nodes in a level and the slot of its first node, for three
+// levels in turn (one being read, the next being filled, the one after zeroed), and the depth so far.
+struct Levels {
+    int count[3], first[3], depth;
+};
+// Starts a level's launch: false when the level is empty for the calling block.  Every launch empties
+// the counter of the level after the next, so a launch past the last level finds nothing and harms
+// nothing, and the host need not wait for the count of each level.
+__device__ __forceinline__ bool beginLevel(Levels* lv, int level) {
+    const int n = lv->count[level % 3];
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        lv->count[(level + 2) % 3] = 0;
+        if (n > 0) {
+            lv->first[(level + 1) % 3] = lv->first[level % 3] + n;
+            lv->depth = level + 1;
+        }
+    }
+    return (int)(blockIdx.x * blockDim.x) < n;
+}
+// Places of this lane's `inner` children in the next level (whole warps call it; one addition per warp).
+__device__ __forceinline__ int placeChildren(Levels* lv, int level, int inner) {
+    const int lane = threadIdx.x & 31;
+    int sum = inner;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += v;
+    }
+    int base = 0;
+    if (lane == 31 && sum > 0) base = atomicAdd(&lv->count[(level + 1) % 3], sum);
+    return __shfl_sync(0xffffffffu, base, 31) + sum - inner;
+}
+__global__ void k_collapse4(const float4* nodes2, const int* frontier, Levels* lv, int level, float4* nodes4, int* next) {
+    if (!beginLevel(lv, level)) return;
+    const int n = lv->count[level % 3], first = lv->first[level % 3];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool valid = i < n;
+    const int item = valid ? frontier[i] : 0;
     Child4 c[4];
     int cnt = 2;
-    readChildren(nodes2, (uint32_t)item.x, c[0], c[1]);
+    readChildren(nodes2, (uint32_t)item, c[0], c[1]);
     while (cnt < 4) {
         int best = -1;
         float bestA = -1.0f;
@@ -630,7 +796,11 @@ __global__ void k_collapse4(const float4* nodes2, const int2* frontier, const in
         c[best] = a;
         c[cnt++] = b;
     }
-    float4* out = nodes4 + 8 * (size_t)item.y;
+    int inner = 0;
+    for (int k = 0; k < cnt; ++k) inner += (c[k].ref & kLeafFlag) ? 0 : 1;
+    int at = placeChildren(lv, level, valid ? inner : 0);
+    if (!valid) return;
+    float4* out = nodes4 + 8 * (size_t)(first + i);
     float v[6][4];
     uint32_t refs[4];
     for (int k = 0; k < 4; ++k) {
@@ -638,9 +808,8 @@ __global__ void k_collapse4(const float4* nodes2, const int2* frontier, const in
             for (int a = 0; a < 3; ++a) { v[2 * a][k] = c[k].lo[a]; v[2 * a + 1][k] = c[k].hi[a]; }
             uint32_t r = c[k].ref;
             if (!(r & kLeafFlag)) {
-                int slot = atomicAdd(nodeCounter, 1);
-                next[atomicAdd(nNext, 1)] = make_int2((int)r, slot);
-                r = (uint32_t)slot;
+                next[at] = (int)r;
+                r = (uint32_t)(first + n + at++);  // the next level's slots follow this level's
             }
             refs[k] = r;
         } else {
@@ -652,38 +821,51 @@ __global__ void k_collapse4(const float4* nodes2, const int2* frontier, const in
     out[6] = make_float4(__uint_as_float(refs[0]), __uint_as_float(refs[1]), __uint_as_float(refs[2]), __uint_as_float(refs[3]));
     out[7] = make_float4(__int_as_float(cnt), 0.0f, 0.0f, 0.0f);
 }
-__global__ void k_collapse_root(int2* frontier, int* nFront, int* nodeCounter) {
-    frontier[0] = make_int2(0, 0);
-    *nFront = 1;
-    *nodeCounter = 1;
+__global__ void k_collapse_root(int* frontier, Levels* lv) {
+    *lv = Levels{{1, 0, 0}, {0, 1, 0}, 0};
+    frontier[0] = 0;
 }
-}  // namespace
 
-size_t bvh4ScratchBytes(int nNodes2) { return 2 * sizeof(int2) * (size_t)std::max(1, nNodes2) + 1024; }
-
-int buildBvh4(const float4* nodes2, int nNodes2, float4* nodes4, void* scratch, int* hostNodeCount, int* hostDepth, cudaStream_t st) {
+// Runs launch(level, bound, ...) for every level.  A level has at most width times the nodes of the one
+// before and at most the binary nodes; the counts are looked at once those bounds meet and then after
+// every third level.
+template <class Launch>
+int buildLevels(int nNodes2, int width, void* scratch, int* hostNodeCount, int* hostDepth, cudaStream_t st, Launch launch) {
     *hostNodeCount = 0;
     *hostDepth = 0;
     if (nNodes2 <= 0) return 0;
-    char* p = static_cast<char*>(scratch);
-    int* counters = reinterpret_cast<int*>(p);  // [0] node counter, [1], [2] frontier sizes
-    int2* fr[2] = {reinterpret_cast<int2*>(p + 256), reinterpret_cast<int2*>(p + 256) + nNodes2};
-    k_collapse_root<<<1, 1, 0, st>>>(fr[0], counters + 1, counters);
-    int cur = 0, depth = 0, n = 1;
-    int hostCnt = 0;
-    while (n > 0) {
-        if (++depth > 4 * kMaxBvhDepth) return -2;
-        if (cudaMemsetAsync(counters + 2 - cur, 0, sizeof(int), st) != cudaSuccess) return -1;
-        k_collapse4<<<(n + 127) / 128, 128, 0, st>>>(nodes2, fr[cur], counters + 1 + cur, nodes4, counters, fr[1 - cur], counters + 2 - cur);
-        if (cudaMemcpyAsync(&n, counters + 2 - cur, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess) return -1;
+    Levels* lv = static_cast<Levels*>(scratch);
+    int* fr[2] = {reinterpret_cast<int*>(static_cast<char*>(scratch) + 256), reinterpret_cast<int*>(static_cast<char*>(scratch) + 256) + nNodes2};
+    k_collapse_root<<<1, 1, 0, st>>>(fr[0], lv);
+    long long bound = 1;
+    int sinceLook = 0;
+    bool looking = false;
+    for (int level = 0; level < 4 * kMaxBvhDepth; ++level) {
+        launch(level, int(bound), lv, fr[level & 1], fr[1 - (level & 1)]);
+        bound = std::min<long long>(bound * width, nNodes2);
+        looking |= bound == nNodes2;
+        if (!looking || ++sinceLook < 3) continue;
+        sinceLook = 0;
+        Levels h;
+        if (cudaMemcpyAsync(&h, lv, sizeof(Levels), cudaMemcpyDeviceToHost, st) != cudaSuccess) return -1;
         if (cudaStreamSynchronize(st) != cudaSuccess) return -1;
-        cur = 1 - cur;
+        bound = h.count[(level + 1) % 3];
+        if (bound == 0) {
+            *hostDepth = h.depth;
+            *hostNodeCount = h.first[h.depth % 3];
+            return 0;
+        }
     }
-    if (cudaMemcpyAsync(&hostCnt, counters, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess) return -1;
-    if (cudaStreamSynchronize(st) != cudaSuccess) return -1;
-    *hostNodeCount = hostCnt;
-    *hostDepth = depth;
-    return 0;
+    return -2;
+}
+}  // namespace
+
+size_t bvh4ScratchBytes(int nNodes2) { return 2 * sizeof(int) * (size_t)std::max(1, nNodes2) + 1024; }
+
+int buildBvh4(const float4* nodes2, int nNodes2, float4* nodes4, void* scratch, int* hostNodeCount, int* hostDepth, cudaStream_t st) {
+    return buildLevels(nNodes2, 4, scratch, hostNodeCount, hostDepth, st, [&](int level, int bound, Levels* lv, int* frontier, int* next) {
+        k_collapse4<<<(bound + 127) / 128, 128, 0, st>>>(nodes2, frontier, lv, level, nodes4, next);
+    });
 }
 }  // namespace sst
 
@@ -703,14 +885,15 @@ int buildBvh4(const float4* nodes2, int nNodes2, float4* nodes4, void* scratch, 
 // =============================================================================================
 namespace sst {
 namespace {
-__global__ void k_collapse8(const float4* nodes2, const int2* frontier, const int* nFront, float4* nodes8, int* nodeCounter, int2* next,
-                            int* nNext) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= *nFront) return;
-    int2 item = frontier[i];
+__global__ void k_collapse8(const float4* nodes2, const int* frontier, Levels* lv, int level, float4* nodes8, int* next) {
+    if (!beginLevel(lv, level)) return;
+    const int n = lv->count[level % 3], first = lv->first[level % 3];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool valid = i < n;
+    const int item = valid ? frontier[i] : 0;
     Child4 c[8];
     int cnt = 2;
-    readChildren(nodes2, (uint32_t)item.x, c[0], c[1]);
+    readChildren(nodes2, (uint32_t)item, c[0], c[1]);
     while (cnt < 8) {
         int best = -1;
         float bestA = -1.0f;
@@ -750,19 +933,22 @@ __global__ void k_collapse8(const float4* nodes2, const int2* frontier, const in
         slotOf[bc] = bs;
         childIn[bs] = bc;
     }
+    int numInner = 0;
+    for (int k = 0; k < cnt; ++k) numInner += (c[k].ref & kLeafFlag) ? 0 : 1;
+    int at = placeChildren(lv, level, valid ? numInner : 0);
+    if (!valid) return;
     float v[6][8];
     uint32_t refs[8];
-    uint32_t valid = 0, inner = 0;
+    uint32_t slots = 0, inner = 0;
     for (int s = 0; s < 8; ++s) {
         const int k = childIn[s];
         if (k >= 0) {
             for (int a = 0; a < 3; ++a) { v[2 * a][s] = c[k].lo[a]; v[2 * a + 1][s] = c[k].hi[a]; }
             uint32_t r = c[k].ref;
-            valid |= 1u << s;
+            slots |= 1u << s;
             if (!(r & kLeafFlag)) {
-                int slot = atomicAdd(nodeCounter, 1);
-                next[atomicAdd(nNext, 1)] = make_int2((int)r, slot);
-                r = (uint32_t)slot;
+                next[at] = (int)r;
+                r = (uint32_t)(first + n + at++);
                 inner |= 1u << s;
             }
             refs[s] = r;
@@ -771,41 +957,22 @@ __global__ void k_collapse8(const float4* nodes2, const int2* frontier, const in
             refs[s] = 0u;
         }
     }
-    float4* out = nodes8 + 15 * (size_t)item.y;
+    float4* out = nodes8 + 15 * (size_t)(first + i);
     for (int a = 0; a < 6; ++a) {
         out[2 * a] = make_float4(v[a][0], v[a][1], v[a][2], v[a][3]);
         out[2 * a + 1] = make_float4(v[a][4], v[a][5], v[a][6], v[a][7]);
     }
     out[12] = make_float4(__uint_as_float(refs[0]), __uint_as_float(refs[1]), __uint_as_float(refs[2]), __uint_as_float(refs[3]));
     out[13] = make_float4(__uint_as_float(refs[4]), __uint_as_float(refs[5]), __uint_as_float(refs[6]), __uint_as_float(refs[7]));
-    out[14] = make_float4(__uint_as_float(valid | (inner << 8)), 0.0f, 0.0f, 0.0f);
+    out[14] = make_float4(__uint_as_float(slots | (inner << 8)), 0.0f, 0.0f, 0.0f);
 }
 }  // namespace
 
-size_t bvh8ScratchBytes(int nNodes2) { return 2 * sizeof(int2) * (size_t)std::max(1, nNodes2) + 1024; }
+size_t bvh8ScratchBytes(int nNodes2) { return bvh4ScratchBytes(nNodes2); }
 
 int buildBvh8(const float4* nodes2, int nNodes2, float4* nodes8, void* scratch, int* hostNodeCount, int* hostDepth, cudaStream_t st) {
-    *hostNodeCount = 0;
-    *hostDepth = 0;
-    if (nNodes2 <= 0) return 0;
-    char* p = static_cast<char*>(scratch);
-    int* counters = reinterpret_cast<int*>(p);  // [0] node counter, [1], [2] frontier sizes
-    int2* fr[2] = {reinterpret_cast<int2*>(p + 256), reinterpret_cast<int2*>(p + 256) + nNodes2};
-    k_collapse_root<<<1, 1, 0, st>>>(fr[0], counters + 1, counters);
-    int cur = 0, depth = 0, n = 1;
-    int hostCnt = 0;
-    while (n > 0) {
-        if (++depth > 4 * kMaxBvhDepth) return -2;
-        if (cudaMemsetAsync(counters + 2 - cur, 0, sizeof(int), st) != cudaSuccess) return -1;
-        k_collapse8<<<(n + 127) / 128, 128, 0, st>>>(nodes2, fr[cur], counters + 1 + cur, nodes8, counters, fr[1 - cur], counters + 2 - cur);
-        if (cudaMemcpyAsync(&n, counters + 2 - cur, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess) return -1;
-        if (cudaStreamSynchronize(st) != cudaSuccess) return -1;
-        cur = 1 - cur;
-    }
-    if (cudaMemcpyAsync(&hostCnt, counters, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess) return -1;
-    if (cudaStreamSynchronize(st) != cudaSuccess) return -1;
-    *hostNodeCount = hostCnt;
-    *hostDepth = depth;
-    return 0;
+    return buildLevels(nNodes2, 8, scratch, hostNodeCount, hostDepth, st, [&](int level, int bound, Levels* lv, int* frontier, int* next) {
+        k_collapse8<<<(bound + 127) / 128, 128, 0, st>>>(nodes2, frontier, lv, level, nodes8, next);
+    });
 }
 }  // namespace sst
