@@ -227,7 +227,7 @@ int sst_autotune(sst_scene* scene, const SstPathTracerParams* params, int32_t tr
  *    process holding the rest of it, where a new allocation can fail in the middle of a frame;
  *  - a caller on a latency-bound loop (shadow or picking queries per frame): cudaFree waits for
  *    the whole device, and cudaMalloc may, which stalls every stream on the GPU, not just this one.
- * The scratch it uses (split ray arrays, queue counters, job record, ray statistics, result flags)
+ * The scratch it uses (rays, work counter, job record, ray statistics, result flags)
  * is one array of 2,361,344 bytes that is part of this library's device code.  Every GPU that
  * loads the library holds it until the process exits.
  * Limits and rules:

@@ -507,6 +507,7 @@ void commitScene(sst_scene* s, int W, int H) {
         d.env.hasCol = s->envHasCol.as<int>();
     }
     d.cam = makeCamera(s->w2c, s->fovDeg, W, H);
+    uploadQueryJob(s);
     CUDA_CHECK(cudaStreamSynchronize(st));
     s->W = W;
     s->H = H;
@@ -531,4 +532,5 @@ void ensureBvh8(sst_scene* s) {
     s->bvh8Depth = depth8;
     s->dev.nodes8 = s->nNodes8 > 0 ? s->nodes8.as<float4>() : nullptr;
     s->dev.nNodes8 = s->nNodes8;
+    uploadQueryJob(s);
 }

@@ -213,8 +213,10 @@ struct sst_ctx {
     WaveStore store[kMaxWaveSets];
     DevBuf stats, film;
     DevBuf chunksBuf, wavesBuf, curWave;
-    // ray queries (sst_trace, sst_occluded): split rays, queue counters, traversal records, results
-    DevBuf qRo, qRd, qCnt, qHits, qOut;
+    // ray queries (sst_trace, sst_occluded): rays, work counter, traversal records, results; the
+    // page-locked record, rays and results of in-place queries
+    DevBuf qRays, qCnt, qHits, qOut;
+    PinnedBuf queryStage;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, evStart = nullptr;
     int* pinnedCount = nullptr;
     // light paths (sst_trace_light_paths)
@@ -365,7 +367,7 @@ void batchJobs(sst_ctx* ctx, const SstRenderJob* jobs, int numJobs, std::vector<
 void batchFilmsOut(sst_ctx* ctx, const SstRenderJob* jobs, int numJobs, const std::vector<JobIn>& in);
 SstRenderStats emptyStats();
 // sst_query.cu
-const DevJob* jobTable(sst_scene* s);
+void uploadQueryJob(sst_scene* s);
 // sst_commit.cu: builds the scene's 8-wide BVH if it has not been built since the last commit.
 void ensureBvh8(sst_scene* s);
 // The context's traversal setting for rays of these scenes: a scene without an 8-wide BVH (not

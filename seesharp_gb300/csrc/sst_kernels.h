@@ -37,8 +37,9 @@ void launch_trace_closest(const TraceTuning& t, const DevJob* jobs, const uint32
                           int* work, float4* hits, DevStats* stats, cudaStream_t s);
 void launch_trace_shadow(const TraceTuning& t, const DevJob* jobs, const uint32_t* rayJob, const float4* ro, const float4* rd, const int* tgt,
                          const int* count, int* work, float4* nee, DevStats* stats, cudaStream_t s);
-void launch_trace_query(const TraceTuning& t, const DevJob* jobs, const float4* ro, const float4* rd, const int* count, int* work, float4* hits,
-                        int* occl, DevStats* stats, bool anyHit, cudaStream_t s);
+// n rays as interleaved records (origin and tmin, direction and tmax), 16-byte aligned.
+void launch_trace_query(const TraceTuning& t, const DevJob* jobs, const float4* rays, int n, int* work, float4* hits, int* occl, DevStats* stats,
+                        bool anyHit, cudaStream_t s);
 // shadeBlocks: the resident blocks per SM of the forward variant with GenericMaterials: the
 // default build (8, 64 registers) or a denser one (10, 12 or 14: 48, 40 or 32 registers, more warps,
 // more spilling); one shadow ray per technique has every build, more shadow rays the default one.

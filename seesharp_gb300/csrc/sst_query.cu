@@ -2,21 +2,30 @@
 // their allocation-free form, and the light-path random walk (LightPathCache.TraceAllPaths).
 #include "sst_host.h"
 
-// A one-entry job table holding the scene (for the ray-query entry points).
-const DevJob* jobTable(sst_scene* s) {
+// The scene's one-entry job table (for the ray-query entry points), uploaded whenever its record
+// changes: at a commit and when the 8-wide BVH is built.
+void uploadQueryJob(sst_scene* s) {
     DevJob j{};
     j.sc = s->dev;
     s->queryJob.ensure(sizeof(DevJob));
     CUDA_CHECK(cudaMemcpyAsync(s->queryJob.p, &j, sizeof(DevJob), cudaMemcpyHostToDevice, s->ctx->stream));
-    return s->queryJob.as<DevJob>();
 }
 
-// Trace / IsOccluded over n rays.  The rays are split into origin and direction arrays and the
-// results written by the device (sst_trace: the SstHit records are expanded on the device from the
-// traversal's (t, u, v, triangle) records); host results come back in one copy.  The buffers are
-// the context's and only grow, so repeated queries of the same size allocate nothing.
+// Queries of up to this many rays between host arrays go through page-locked memory that the kernels
+// read and write in place, instead of two copies.  Closest hits of 97 / 1024 / 2048 / 4096 rays on the
+// Cornell box: 38 / 48 / 51 / 60 us with copies, 33 / 40 / 47 / 63 us in place (its 48-byte records
+// make the link the bound from there on); occlusion of 97 / 4096 / 8192 / 16384 rays: 32 / 43 / 44 / 46
+// against 25 / 33 / 38 / 51 us.  (65 to 101 us before, with the rays split by two strided copies and the
+// job table, the counters and the statistics uploaded and read back each time.)
+constexpr int kTraceInPlace = 2048, kOcclInPlace = 8192;
+
+// Trace / IsOccluded over n rays.  The traversal reads the SstRay records where they are (device
+// arrays on a 16-byte boundary) or from one copy of them; sst_trace's SstHit records are expanded on the
+// device from the traversal's (t, u, v, triangle) records.  The buffers are the context's and only
+// grow, so repeated queries of the same size allocate nothing.
 static void runQuery(sst_scene* s, const SstRay* rays, int n, SstHit* hits, int32_t* occl, int memory, bool anyHit) {
     static_assert(sizeof(SstHit) == sizeof(SstHitDev), "hit layout");
+    static_assert(sizeof(SstRay) == 2 * sizeof(float4), "ray layout");
     if (!s || (n > 0 && !rays) || n < 0) fail(SST_ERR_INVALID_ARGUMENT, "invalid query");
     if (memory != SST_MEM_HOST && memory != SST_MEM_DEVICE) fail(SST_ERR_INVALID_ARGUMENT, "memory must be SST_MEM_HOST or SST_MEM_DEVICE");
     if (!s->committed) fail(SST_ERR_NOT_COMMITTED, "scene is not committed");
@@ -24,48 +33,45 @@ static void runQuery(sst_scene* s, const SstRay* rays, int n, SstHit* hits, int3
     sst_ctx* c = s->ctx;
     CUDA_CHECK(cudaSetDevice(c->device));
     cudaStream_t st = c->stream;
-    const cudaMemcpyKind in = memory == SST_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-    const cudaMemcpyKind out = memory == SST_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-    // separate origin / direction arrays (SstRay = org, tmin, dir, tmax = two float4)
-    c->qRo.ensure(size_t(n) * 16);
-    c->qRd.ensure(size_t(n) * 16);
-    CUDA_CHECK(cudaMemcpy2DAsync(c->qRo.p, 16, rays, 32, 16, size_t(n), in, st));
-    CUDA_CHECK(cudaMemcpy2DAsync(c->qRd.p, 16, reinterpret_cast<const char*>(rays) + 16, 32, 16, size_t(n), in, st));
-    c->qCnt.ensure(sizeof(int) * 2);
-    c->pinnedCount[0] = n;
-    c->pinnedCount[1] = 0;
-    CUDA_CHECK(cudaMemcpyAsync(c->qCnt.p, c->pinnedCount, sizeof(int) * 2, cudaMemcpyHostToDevice, st));
-    c->stats.ensure(sizeof(DevStats));
-    CUDA_CHECK(cudaMemsetAsync(c->stats.p, 0, sizeof(DevStats), st));
-    int* cnt = c->qCnt.as<int>();
-    if (anyHit) {
-        int* dOcc = occl;
-        if (memory != SST_MEM_DEVICE) {
-            c->qOut.ensure(size_t(n) * 4);
-            dOcc = c->qOut.as<int>();
-        }
-        const TraceTuning tt = traceForBuilding(c, &s, 1);
-        launch_trace_query(tt, jobTable(s), c->qRo.as<float4>(), c->qRd.as<float4>(), cnt, cnt + 1, nullptr, dOcc, c->stats.as<DevStats>(), true, st);
-        CUDA_CHECK(cudaGetLastError());
-        if (memory != SST_MEM_DEVICE) CUDA_CHECK(cudaMemcpyAsync(occl, dOcc, size_t(n) * 4, out, st));
+    const bool device = memory == SST_MEM_DEVICE, inPlace = !device && n <= (anyHit ? kOcclInPlace : kTraceInPlace);
+    const size_t rayBytes = size_t(n) * sizeof(SstRay), outBytes = size_t(n) * (anyHit ? sizeof(int32_t) : sizeof(SstHitDev));
+    void* const userOut = anyHit ? static_cast<void*>(occl) : static_cast<void*>(hits);
+    const TraceTuning tt = traceForBuilding(c, &s, 1);
+    // page-locked: the overflow flag's record, then the rays and results of an in-place query
+    c->queryStage.ensure(256 + size_t(kOcclInPlace) * (sizeof(SstRay) + sizeof(int32_t)));
+    static_assert(size_t(kTraceInPlace) * (sizeof(SstRay) + sizeof(SstHitDev)) <= size_t(kOcclInPlace) * (sizeof(SstRay) + sizeof(int32_t)), "stage size");
+    char* const stage = c->queryStage.as<char>();
+    DevStats* const stats = reinterpret_cast<DevStats*>(stage);
+    static_assert(sizeof(DevStats) <= 256, "query stage layout");
+    std::memset(stats, 0, sizeof(DevStats));
+    const void* dRays = rays;
+    void* dOut = userOut;
+    if (inPlace) {
+        std::memcpy(stage + 256, rays, rayBytes);
+        dRays = stage + 256;
+        dOut = stage + 256 + rayBytes;
     } else {
-        c->qHits.ensure(size_t(n) * 16);
-        const TraceTuning tt = traceForBuilding(c, &s, 1);
-        launch_trace_query(tt, jobTable(s), c->qRo.as<float4>(), c->qRd.as<float4>(), cnt, cnt + 1, c->qHits.as<float4>(), nullptr, c->stats.as<DevStats>(),
-                           false, st);
-        SstHitDev* dHits = reinterpret_cast<SstHitDev*>(hits);
-        if (memory != SST_MEM_DEVICE) {
-            c->qOut.ensure(size_t(n) * sizeof(SstHitDev));
-            dHits = c->qOut.as<SstHitDev>();
+        if (!device || (reinterpret_cast<uintptr_t>(rays) & 15u)) {
+            c->qRays.ensure(rayBytes);
+            CUDA_CHECK(cudaMemcpyAsync(c->qRays.p, rays, rayBytes, device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
+            dRays = c->qRays.p;
         }
-        launch_hit_expand(s->dev, c->qHits.as<float4>(), n, dHits, st);
-        CUDA_CHECK(cudaGetLastError());
-        if (memory != SST_MEM_DEVICE) CUDA_CHECK(cudaMemcpyAsync(hits, dHits, size_t(n) * sizeof(SstHitDev), out, st));
+        if (!device) {
+            c->qOut.ensure(outBytes);
+            dOut = c->qOut.p;
+        }
     }
-    DevStats hs;
-    CUDA_CHECK(cudaMemcpyAsync(&hs, c->stats.p, sizeof(DevStats), cudaMemcpyDeviceToHost, st));
+    c->qCnt.ensure(sizeof(int));
+    CUDA_CHECK(cudaMemsetAsync(c->qCnt.p, 0, sizeof(int), st));
+    if (!anyHit) c->qHits.ensure(size_t(n) * 16);
+    launch_trace_query(tt, s->queryJob.as<DevJob>(), static_cast<const float4*>(dRays), n, c->qCnt.as<int>(), c->qHits.as<float4>(),
+                       static_cast<int*>(dOut), stats, anyHit, st);
+    if (!anyHit) launch_hit_expand(s->dev, c->qHits.as<float4>(), n, static_cast<SstHitDev*>(dOut), st);
+    CUDA_CHECK(cudaGetLastError());
+    if (!device && !inPlace) CUDA_CHECK(cudaMemcpyAsync(userOut, dOut, outBytes, cudaMemcpyDeviceToHost, st));
     CUDA_CHECK(cudaStreamSynchronize(st));
-    if (hs.errorFlags & 1) fail(SST_ERR_DEVICE_LIMIT, "BVH traversal stack overflow");
+    if (stats->errorFlags & 1) fail(SST_ERR_DEVICE_LIMIT, "BVH traversal stack overflow");
+    if (inPlace) std::memcpy(userOut, dOut, outBytes);
 }
 
 static LightPathBuf bindLight(DevBuf* b, size_t cap) {
@@ -131,7 +137,7 @@ int sst_trace_light_paths(sst_scene* s, uint32_t seed, uint32_t iteration, int32
         c->stats.ensure(sizeof(DevStats));
         CUDA_CHECK(cudaMemsetAsync(c->stats.p, 0, sizeof(DevStats), st));
         const TraceTuning tt = traceForBuilding(c, &s, 1);
-        const DevJob* job = jobTable(s);
+        const DevJob* job = s->queryJob.as<DevJob>();
         LightParams P{numPaths, maxDepth, seed, iteration};
         CUDA_CHECK(cudaEventRecord(c->ev0, st));
         launch_light_start(job, P, A, cnt, dv, dl, st);
@@ -173,11 +179,10 @@ int sst_trace_light_paths(sst_scene* s, uint32_t seed, uint32_t iteration, int32
 // ---------------------------------------------------------------------------------------------
 // Allocation-free occlusion query (sst_occluded_noalloc).  Its scratch is one array of fixed size
 // in this library's device image, laid out as
-//   [0, 256)      queue length and work counter of the traversal kernel
+//   [0, 256)      work counter of the traversal kernel
 //   [256, 512)    DevStats (ray counts)
 //   [512, 2048)   DevJob (the scene record the traversal kernel reads)
-//   then          ray origins (float4 x max rays), ray directions (float4 x max rays),
-//                 occlusion flags (int x max rays).
+//   then          rays (two float4 x max rays), occlusion flags (int x max rays).
 // ---------------------------------------------------------------------------------------------
 namespace {
 constexpr size_t kNaCounters = 0, kNaStats = 256, kNaJob = 512, kNaHeader = 2048;
@@ -223,22 +228,17 @@ extern "C" int sst_occluded_noalloc(sst_scene* s, const SstRay* rays, int32_t n,
         int* cnt = reinterpret_cast<int*>(base + kNaCounters);
         DevStats* stats = reinterpret_cast<DevStats*>(base + kNaStats);
         DevJob* job = reinterpret_cast<DevJob*>(base + kNaJob);
-        float4* ro = reinterpret_cast<float4*>(base + kNaHeader);
-        float4* rd = ro + kNaMaxRays;
-        int* occ = reinterpret_cast<int*>(rd + kNaMaxRays);
+        float4* dRays = reinterpret_cast<float4*>(base + kNaHeader);
+        int* occ = reinterpret_cast<int*>(dRays + 2 * kNaMaxRays);
         const cudaMemcpyKind in = memory == SST_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
         const cudaMemcpyKind out = memory == SST_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-        // SstRay = {org, tmin, dir, tmax}: split into the origin and direction arrays
-        CUDA_CHECK(cudaMemcpy2DAsync(ro, 16, rays, 32, 16, size_t(n), in, st));
-        CUDA_CHECK(cudaMemcpy2DAsync(rd, 16, reinterpret_cast<const char*>(rays) + 16, 32, 16, size_t(n), in, st));
-        // set every call: the queue length (n), the work counter and the statistics (zero), the job
-        const int hostCnt[2] = {n, 0};
-        CUDA_CHECK(cudaMemcpyAsync(cnt, hostCnt, sizeof(hostCnt), cudaMemcpyHostToDevice, st));
-        CUDA_CHECK(cudaMemsetAsync(stats, 0, sizeof(DevStats), st));
+        CUDA_CHECK(cudaMemcpyAsync(dRays, rays, size_t(n) * sizeof(SstRay), in, st));
+        // set every call: the work counter and the statistics (zero), the job
+        CUDA_CHECK(cudaMemsetAsync(base, 0, kNaJob, st));
         DevJob j{};
         j.sc = s->dev;
         CUDA_CHECK(cudaMemcpyAsync(job, &j, sizeof(DevJob), cudaMemcpyHostToDevice, st));
-        launch_trace_query(traceFor(c, &s, 1), job, ro, rd, cnt, cnt + 1, nullptr, occ, stats, true, st);
+        launch_trace_query(traceFor(c, &s, 1), job, dRays, n, cnt, nullptr, occ, stats, true, st);
         CUDA_CHECK(cudaGetLastError());
         CUDA_CHECK(cudaMemcpyAsync(occluded, occ, size_t(n) * 4, out, st));
         CUDA_CHECK(cudaStreamSynchronize(st));

@@ -496,6 +496,8 @@ template <> struct WideTrav<8> {
     SST_D static bool run(State& s, int* sstack, int* lstack, int* err, int pause) { return trav8Run<ANY, BLOCK, SSTACK>(s, sstack, lstack, err, pause); }
 };
 
+// The rays are count's (or nRays of them, when count is null), ray i at ro[i * rayStride] and
+// rd[i * rayStride]: two arrays (stride 1) or one of interleaved records (stride 2).
 // mode 0: closest hit -> hits[i]; mode 1: shadow rays, zero nee[tgt[i]] when occluded;
 // mode 2: any hit -> occl[i] = 1/0.
 // Resident threads per SM the traversal kernels are compiled for (register budget); 0: no bound.
@@ -513,9 +515,9 @@ template <int MODE, int BLOCK, int SSTACK, int W>
 __global__ void __launch_bounds__(BLOCK, (W == 8 ? SST_TRACE8_MIN_THREADS : SST_TRACE_MIN_THREADS) > 0
                                              ? (W == 8 ? SST_TRACE8_MIN_THREADS : SST_TRACE_MIN_THREADS) / BLOCK : 1) k_trace(const DevJob* __restrict__ jobs, const uint32_t* __restrict__ rayJob, const float4* ro,
                                                  const float4* rd, const int* count, int* work, float4* hits, const int* tgt, float4* nee,
-                                                 int* occl, DevStats* stats, int countRays, int refillIdle) {
+                                                 int* occl, DevStats* stats, int countRays, int refillIdle, int nRays, int rayStride) {
     __shared__ int sstack[SSTACK * BLOCK];
-    const int n = *count;
+    const int n = count ? *count : nRays;
     const int lane = threadIdx.x & 31;
     if (countRays && blockIdx.x == 0 && threadIdx.x == 0) {
         if (MODE == 0) atomicAdd(&stats->rays, (unsigned long long)n);
@@ -542,7 +544,7 @@ __global__ void __launch_bounds__(BLOCK, (W == 8 ? SST_TRACE8_MIN_THREADS : SST_
                     const int j = base + __popc(idle & ((1u << lane) - 1u));
                     if (j < n) {
                         i = j;
-                        const float4 o = ro[j], d = rd[j];
+                        const float4 o = ro[(size_t)j * rayStride], d = rd[(size_t)j * rayStride];
                         const uint32_t jb = rayJob ? rayJob[j] : 0u;
                         T::begin(s, jobs[jb].sc, f3(o), f3(d), o.w, d.w);
                     }
@@ -568,7 +570,7 @@ __global__ void __launch_bounds__(BLOCK, (W == 8 ? SST_TRACE8_MIN_THREADS : SST_
         if (base >= n) break;
         int i = base + lane;
         if (i < n) {
-            float4 o = ro[i], d = rd[i];
+            float4 o = ro[(size_t)i * rayStride], d = rd[(size_t)i * rayStride];
             uint32_t jb = rayJob ? rayJob[i] : 0u;
             const DevScene& sc = jobs[jb].sc;
             TraceResult h = traverse<MODE != 0, BLOCK, SSTACK>(bvhOf(sc), f3(o), f3(d), o.w, d.w, sstack, &stats->errorFlags);
@@ -588,7 +590,7 @@ __global__ void __launch_bounds__(BLOCK, (W == 8 ? SST_TRACE8_MIN_THREADS : SST_
 // Variant table: BVH width x block size x shared stack entries, for each of the three modes.
 // ---------------------------------------------------------------------------------------------
 using TraceKernel = void (*)(const DevJob*, const uint32_t*, const float4*, const float4*, const int*, int*, float4*, const int*, float4*, int*,
-                             DevStats*, int, int);
+                             DevStats*, int, int, int, int);
 
 template <int BLOCK, int SSTACK, int W>
 struct TraceVariant {
@@ -696,26 +698,32 @@ int traceMaxBlocksPerSM(const TraceTuning& t) {
     return maxBlocksPerSM(v < 0 ? 4 : v);
 }
 
+// nRays: the number of rays where the host knows it (count is null then), which also bounds the grid: a
+// block takes its first rays 32 per warp, so more blocks than that would only start and end.
 static void launch(const TraceTuning& t, int mode, const DevJob* jobs, const uint32_t* rayJob, const float4* ro, const float4* rd, const int* count,
-                   int* work, float4* hits, const int* tgt, float4* nee, int* occl, DevStats* stats, int countRays, cudaStream_t s) {
+                   int* work, float4* hits, const int* tgt, float4* nee, int* occl, DevStats* stats, int countRays, int nRays, int rayStride,
+                   cudaStream_t s) {
     int v = variantOf(t);
     if (v < 0) v = 4;  // 128 threads, 24 shared entries, binary
-    traceKernel(mode, v)<<<traceGrid(t), kBlocks[(v % 9) / 3], 0, s>>>(jobs, rayJob, ro, rd, count, work, hits, tgt, nee, occl, stats, countRays,
-                                                                        t.refillIdle);
+    const int block = kBlocks[(v % 9) / 3];
+    int grid = traceGrid(t);
+    if (!count) grid = std::min(grid, (nRays + block - 1) / block);
+    traceKernel(mode, v)<<<grid, block, 0, s>>>(jobs, rayJob, ro, rd, count, work, hits, tgt, nee, occl, stats, countRays, t.refillIdle, nRays, rayStride);
 }
 
 void launch_trace_closest(const TraceTuning& t, const DevJob* jobs, const uint32_t* rayJob, const float4* ro, const float4* rd, const int* count,
                           int* work, float4* hits, DevStats* stats, cudaStream_t s) {
-    launch(t, 0, jobs, rayJob, ro, rd, count, work, hits, nullptr, nullptr, nullptr, stats, 1, s);
+    launch(t, 0, jobs, rayJob, ro, rd, count, work, hits, nullptr, nullptr, nullptr, stats, 1, 0, 1, s);
 }
 void launch_trace_shadow(const TraceTuning& t, const DevJob* jobs, const uint32_t* rayJob, const float4* ro, const float4* rd, const int* tgt,
                          const int* count, int* work, float4* nee, DevStats* stats, cudaStream_t s) {
-    launch(t, 1, jobs, rayJob, ro, rd, count, work, nullptr, tgt, nee, nullptr, stats, 0, s);
+    launch(t, 1, jobs, rayJob, ro, rd, count, work, nullptr, tgt, nee, nullptr, stats, 0, 0, 1, s);
 }
-void launch_trace_query(const TraceTuning& t, const DevJob* jobs, const float4* ro, const float4* rd, const int* count, int* work, float4* hits,
-                        int* occl, DevStats* stats, bool anyHit, cudaStream_t s) {
-    if (anyHit) launch(t, 2, jobs, nullptr, ro, rd, count, work, nullptr, nullptr, nullptr, occl, stats, 0, s);
-    else launch(t, 0, jobs, nullptr, ro, rd, count, work, hits, nullptr, nullptr, nullptr, stats, 0, s);
+void launch_trace_query(const TraceTuning& t, const DevJob* jobs, const float4* rays, int n, int* work, float4* hits, int* occl, DevStats* stats,
+                        bool anyHit, cudaStream_t s) {
+    if (n <= 0) return;
+    launch(t, anyHit ? 2 : 0, jobs, nullptr, rays, rays + 1, nullptr, work, anyHit ? nullptr : hits, nullptr, nullptr, anyHit ? occl : nullptr, stats, 0, n, 2,
+           s);
 }
 
 }  // namespace sst
