@@ -185,13 +185,12 @@ struct BatchSig {
 };
 
 // One set of wavefront buffers: path state (A and B), hits, next-event slots, shadow-ray queue,
-// counters, shade order, per-item path estimates, the split shade form's record, the denoiser
-// feature samples and the job table that points at them.  The context keeps kMaxWaveSets, so
-// that that many waves can be in flight.
+// counters, shade order, per-item path estimates, the split shade form's record and the denoiser
+// feature samples.  The context keeps kMaxWaveSets, so that that many waves can be in flight.
 constexpr int kMaxWaveSets = 3;
 struct WaveStore {
     DevBuf pathA[10], pathB[10];
-    DevBuf hits, nee, shRo, shRd, shTgt, shJob, counters, order, samples, rec, aov, jobs;
+    DevBuf hits, nee, shRo, shRd, shTgt, shJob, counters, order, samples, rec, aov;
     DevBuf adjA[3], adjB[3], neeG;  // the adjoint replay's per-path state and next-event payloads
     int cap = 0, neeSlots = 0;
     // its streams: the bounces (and, with one wave in flight, everything) run on `run`, a bounce's
@@ -212,7 +211,9 @@ struct sst_ctx {
     // wavefront buffers (store[1..] only while several waves are in flight)
     WaveStore store[kMaxWaveSets];
     DevBuf stats, film;
-    DevBuf chunksBuf, wavesBuf, curWave;
+    // a render's tables (statistics, wave indices, waves, chunks, job tables) and their page-locked copy
+    DevBuf renderBlock;
+    PinnedBuf renderStage;
     // ray queries (sst_trace, sst_occluded): rays, work counter, traversal records, results; the
     // page-locked record, rays and results of in-place queries
     DevBuf qRays, qCnt, qHits, qOut;
@@ -222,7 +223,8 @@ struct sst_ctx {
     // light paths (sst_trace_light_paths)
     DevBuf lightA[9], lightB[9], lightHits, lightVerts, lightLengths, lightCnt;
     // frame-buffer layers (sst_render_layers)
-    DevBuf layMean, layRef, layErr, layVar, laySum, layAlb, layNrm, layErrPix, layTrim, layOutW, layOutIt, layPyr, pyrG;
+    DevBuf layBlock, layRef, layErr, layVar, laySum, layErrPix, layTrim, layPyr, pyrG;
+    PinnedBuf layStage;
     // batched adjoint: the jobs of the last sst_forward_batch, their path radiance, dLoss/dImage
     std::vector<BatchSig> batchSig;
     std::vector<std::unique_ptr<DevBuf>> batchRecord, batchDLdI;
@@ -360,7 +362,8 @@ void commitScene(sst_scene* s, int W, int H);
 int defaultWaveCapacity();
 void ensureWave(sst_ctx* c, int cap, int ns, Wave& w, int set);
 void checkParams(const sst_scene* s, const SstPathTracerParams* p);
-void renderJobs(sst_ctx* c, std::vector<JobIn>& jobs, SstRenderStats* out, bool replay = false, const std::vector<WaveChunk>* paths = nullptr);
+void renderJobs(sst_ctx* c, std::vector<JobIn>& jobs, SstRenderStats* out, bool replay = false, const std::vector<WaveChunk>* paths = nullptr,
+                HostPrefault* prefault = nullptr);
 size_t texPoolFloats(const sst_scene* s);
 void batchJobs(sst_ctx* ctx, const SstRenderJob* jobs, int numJobs, std::vector<JobIn>& in, std::vector<std::unique_ptr<DevBuf>>& staged,
                bool fromZero);

@@ -52,7 +52,6 @@ void ensureWave(sst_ctx* c, int cap, int ns, Wave& w, int set) {
     ws.shJob.ensure(shCap * 4);
     ws.counters.ensure(sizeof(int) * kNumCounters);
     ws.order.ensure(size_t(ws.cap) * 4);
-    c->stats.ensure(sizeof(DevStats));
     w.wb.hits = ws.hits.as<float4>();
     w.wb.nee = ws.nee.as<float4>();
     w.wb.shRo = ws.shRo.as<float4>();
@@ -127,7 +126,8 @@ static void planWaves(std::vector<JobIn>& jobs, int cap, bool iterationPerWave, 
 // paths: instead of the jobs' iteration ranges, render exactly these single-path chunks (one
 // (pixel, iteration) each, at most one wave) without folding them into a film; each path's
 // estimate is left in the first buffer set's samples at its chunk's item offset.
-void renderJobs(sst_ctx* c, std::vector<JobIn>& jobs, SstRenderStats* out, bool replay, const std::vector<WaveChunk>* paths) {
+// prefault: started after the first wave's launches (the caller finishes it).
+void renderJobs(sst_ctx* c, std::vector<JobIn>& jobs, SstRenderStats* out, bool replay, const std::vector<WaveChunk>* paths, HostPrefault* prefault) {
     cudaStream_t st = c->stream;
     if (jobs.empty()) return;
     long long totalItems = 0;
@@ -232,34 +232,49 @@ void renderJobs(sst_ctx* c, std::vector<JobIn>& jobs, SstRenderStats* out, bool 
         if (replay) bindAdj(ws[k], k);
         c->store[k].samples.ensure(size_t(ws[k].wb.cap) * 12);
     }
+    // What the kernels read besides the paths, in one device block uploaded by one copy (from
+    // page-locked memory unless it is a large path list): the statistics (zero), the wave indices ([0]
+    // the wave being folded, [1] the fold's finished-block count, [2 + 2s] the wave whose bounces buffer
+    // set s runs), the waves, their chunks, and a job table per buffer set, which points at the denoiser
+    // feature samples of the set's waves.  As seven uploads and clears with a wait, and a thread started before them, the 160 x 90 preview
+    // spent 163 us before its first kernel (traced), 66 us now.
+    auto place = [](size_t& end, size_t bytes) {
+        const size_t at = (end + 255) & ~size_t(255);
+        end = at + bytes;
+        return at;
+    };
+    size_t blockBytes = 0;
+    const size_t oStats = place(blockBytes, sizeof(DevStats)), oCur = place(blockBytes, sizeof(int) * (2 + 2 * kMaxWaveSets));
+    const size_t oWaves = place(blockBytes, waves.size() * sizeof(WaveDesc)), oChunks = place(blockBytes, chunks.size() * sizeof(WaveChunk));
+    size_t oJobs[kMaxWaveSets];
+    for (int k = 0; k < nSets; ++k) oJobs[k] = place(blockBytes, hj.size() * sizeof(DevJob));
+    c->renderBlock.ensure(blockBytes);
+    const bool staged = blockBytes <= (size_t(1) << 20);
+    c->renderStage.ensure(staged ? size_t(1) << 20 : sizeof(DevStats));
+    std::vector<char> pageable(staged ? 0 : blockBytes);
+    char* const hostBlock = staged ? c->renderStage.as<char>() : pageable.data();
+    std::memset(hostBlock + oStats, 0, sizeof(DevStats));
+    for (int k = 0; k < 2 + 2 * kMaxWaveSets; ++k) reinterpret_cast<int*>(hostBlock + oCur)[k] = k >= 2 && k % 2 == 0 ? (k - 2) / 2 : 0;
+    std::memcpy(hostBlock + oWaves, waves.data(), waves.size() * sizeof(WaveDesc));
+    std::memcpy(hostBlock + oChunks, chunks.data(), chunks.size() * sizeof(WaveChunk));
+    const DevJob* setJobs[kMaxWaveSets] = {};
     for (int k = 0; k < nSets; ++k) {
         // sized by the set's own capacity (the sets grow separately), which indexes them
         WaveStore& sk = c->store[k];
         if (anyAov) sk.aov.ensure(size_t(ws[k].wb.cap) * 24);
         if (split) sk.rec.ensure(size_t(kShadeRec) * size_t(ws[k].wb.cap) * 16);
-        // the set's job table (its own host copy, so that no upload depends on when the copy of the
-        // host vector completes): the denoiser feature samples of its waves
-        std::vector<DevJob> hs = hj;
-        for (auto& j : hs)
-            if (j.lay.aovAlbedo) j.lay.aovSamples = sk.aov.as<float>();
-        sk.jobs.upload(hs, st);
-        CUDA_CHECK(cudaStreamSynchronize(st));
+        DevJob* const tab = reinterpret_cast<DevJob*>(hostBlock + oJobs[k]);
+        std::memcpy(tab, hj.data(), hj.size() * sizeof(DevJob));
+        for (size_t j = 0; j < hj.size(); ++j)
+            if (tab[j].lay.aovAlbedo) tab[j].lay.aovSamples = sk.aov.as<float>();
+        setJobs[k] = reinterpret_cast<const DevJob*>(c->renderBlock.as<char>() + oJobs[k]);
     }
-    c->chunksBuf.upload(chunks, st);
-    c->wavesBuf.upload(waves, st);
-    // wave indices: [0] the wave being folded, [1] the fold's finished-block count, [2 + 2s] the wave
-    // whose bounces buffer set s runs (several waves in flight)
-    c->curWave.ensure(sizeof(int) * (2 + 2 * kMaxWaveSets));
-    {
-        int init[2 + 2 * kMaxWaveSets] = {};
-        for (int k = 0; k < kMaxWaveSets; ++k) init[2 + 2 * k] = k;
-        CUDA_CHECK(cudaMemcpyAsync(c->curWave.p, init, sizeof(init), cudaMemcpyHostToDevice, st));
-    }
-    const WaveChunk* dch = c->chunksBuf.as<WaveChunk>();
-    const WaveDesc* dwv = c->wavesBuf.as<WaveDesc>();
-    int* dcur = c->curWave.as<int>();
-    DevStats* dstats = c->stats.as<DevStats>();
-    CUDA_CHECK(cudaMemsetAsync(dstats, 0, sizeof(DevStats), st));
+    CUDA_CHECK(cudaMemcpyAsync(c->renderBlock.p, hostBlock, blockBytes, cudaMemcpyHostToDevice, st));
+    if (!staged) CUDA_CHECK(cudaStreamSynchronize(st));
+    const WaveChunk* dch = reinterpret_cast<const WaveChunk*>(c->renderBlock.as<char>() + oChunks);
+    const WaveDesc* dwv = reinterpret_cast<const WaveDesc*>(c->renderBlock.as<char>() + oWaves);
+    int* dcur = reinterpret_cast<int*>(c->renderBlock.as<char>() + oCur);
+    DevStats* dstats = reinterpret_cast<DevStats*>(c->renderBlock.as<char>() + oStats);
     int maxFold = 0;
     for (auto& wd : waves) maxFold = std::max(maxFold, wd.foldThreads);
 
@@ -270,11 +285,15 @@ void renderJobs(sst_ctx* c, std::vector<JobIn>& jobs, SstRenderStats* out, bool 
     // by the other's blocks), and the next shade waits for them.  Kernel timing (profiling) keeps
     // every launch on the one stream.  camWave: the wave index the camera (and the pyramid) read.
     const bool overlap = !c->profiling;
+    auto launched = [&] {
+        if (prefault) prefault->start();
+        prefault = nullptr;
+    };
     long long launches = 0;  // kernels issued (in graph mode: the nodes of one wave)
     auto issueWave = [&](int set, cudaStream_t rs, int items, bool allowEarlyExit, bool fold, int* camWave) {
         const WaveBuffers& wb = ws[set].wb;
         WaveStore& sk = c->store[set];
-        const DevJob* dj = sk.jobs.as<DevJob>();
+        const DevJob* dj = setJobs[set];
         float* samples = sk.samples.as<float>();
         launches += fold ? 2 : 1;  // camera and film fold
         int* cnt = wb.counters;
@@ -346,6 +365,7 @@ void renderJobs(sst_ctx* c, std::vector<JobIn>& jobs, SstRenderStats* out, bool 
             if (allowEarlyExit && d >= 6 && d < maxDepth) {
                 // stop early once the queue is empty (long MaxDepth with Russian roulette)
                 CUDA_CHECK(cudaMemcpyAsync(c->pinnedCount, cnt + kCntQueue + d + 1, sizeof(int), cudaMemcpyDeviceToHost, rs));
+                launched();
                 CUDA_CHECK(cudaStreamSynchronize(rs));
                 if (*c->pinnedCount == 0) break;
                 maxItems = *c->pinnedCount;
@@ -404,8 +424,9 @@ void renderJobs(sst_ctx* c, std::vector<JobIn>& jobs, SstRenderStats* out, bool 
             CUDA_CHECK(cudaGraphLaunch(gr.e[set], sk.run));
             CUDA_CHECK(cudaEventRecord(sk.evDone, sk.run));
             CUDA_CHECK(cudaStreamWaitEvent(st, sk.evDone, 0));
-            launch_film_fold(sk.jobs.as<DevJob>(), dch, dwv, dcur, replay ? nullptr : sk.samples.as<float>(), dstats, maxFold, 1, st);
+            launch_film_fold(setJobs[set], dch, dwv, dcur, replay ? nullptr : sk.samples.as<float>(), dstats, maxFold, 1, st);
             CUDA_CHECK(cudaEventRecord(sk.evFolded, st));
+            launched();
         }
         launches = (perWave + 1) * (long long)waves.size();
         CUDA_CHECK(cudaGetLastError());
@@ -425,6 +446,7 @@ void renderJobs(sst_ctx* c, std::vector<JobIn>& jobs, SstRenderStats* out, bool 
         CUDA_CHECK(cudaStreamEndCapture(st, &graph));
         CUDA_CHECK(cudaGraphInstantiate(&exec, graph, 0));
         for (size_t k = 0; k < waves.size(); ++k) CUDA_CHECK(cudaGraphLaunch(exec, st));
+        launched();
         launches *= (long long)waves.size();
         CUDA_CHECK(cudaGetLastError());
         CUDA_CHECK(cudaStreamSynchronize(st));
@@ -440,6 +462,7 @@ void renderJobs(sst_ctx* c, std::vector<JobIn>& jobs, SstRenderStats* out, bool 
                 if (ms + per > double(jobs[0].p.maximumRenderTimeMs)) break;  // PathTracer.cs:221-227
             }
             issueWave(0, st, waves[k].items, true, true, dcur);
+            launched();
             CUDA_CHECK(cudaGetLastError());
             if (c->profiling) {
                 std::vector<int> hc(kNumCounters);
@@ -457,11 +480,11 @@ void renderJobs(sst_ctx* c, std::vector<JobIn>& jobs, SstRenderStats* out, bool 
         }
     }
     CUDA_CHECK(cudaEventRecord(c->ev1, st));
+    CUDA_CHECK(cudaMemcpyAsync(c->renderStage.p, dstats, sizeof(DevStats), cudaMemcpyDeviceToHost, st));
     CUDA_CHECK(cudaStreamSynchronize(st));
+    const DevStats hs = *c->renderStage.as<DevStats>();
     float ms = 0;
     CUDA_CHECK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
-    DevStats hs;
-    CUDA_CHECK(cudaMemcpy(&hs, dstats, sizeof(DevStats), cudaMemcpyDeviceToHost));
     if (hs.errorFlags & 1) fail(SST_ERR_DEVICE_LIMIT, "BVH traversal stack overflow");
     // iterations completed per job
     for (int k = 0; k < wavesDone; ++k)
@@ -550,6 +573,8 @@ SstRenderStats emptyStats() {
     return t;
 }
 
+constexpr size_t kLayStageBytes = size_t(1) << 17;
+
 static TraceTuning toTrace(const SstTuning& t) { return TraceTuning{t.traceBlock, t.traceStackShared, t.traceBlocksPerSM, t.traceBvhWidth, t.traceRefillIdle}; }
 
 static void checkTuning(const SstTuning& t) {
@@ -604,7 +629,6 @@ int sst_render(sst_scene* s, const SstPathTracerParams* p, float* film, int32_t 
         double fbMs = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - tfb0).count();
         HostPrefault prefault;
         if (memory != SST_MEM_DEVICE) prefault.add(film, filmBytes);
-        prefault.start();
         if (p->firstIteration < p->totalSpp) {
             std::vector<JobIn> jobs(1);
             jobs[0].s = s;
@@ -612,7 +636,7 @@ int sst_render(sst_scene* s, const SstPathTracerParams* p, float* film, int32_t 
             jobs[0].dFilm = dFilm;
             jobs[0].iterFirst = p->firstIteration;
             jobs[0].iterEnd = p->totalSpp;
-            renderJobs(c, jobs, &local);
+            renderJobs(c, jobs, &local, false, nullptr, &prefault);
         }
         prefault.finish();
         auto tfb1 = std::chrono::steady_clock::now();
@@ -854,13 +878,30 @@ int sst_render_layers(sst_scene* s, const SstPathTracerParams* p, float* film, i
         const cudaMemcpyKind in = L->memory == SST_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
         const cudaMemcpyKind out = L->memory == SST_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
         SstRenderStats local = emptyStats();
+        // The film (unless it is a device array) and the layers' state share one block: one clear for all
+        // of them, and one read-back for a small image.  Sections: film, variance means and moments,
+        // albedo, normal, outlier priorities; then the outliers' iterations, whose empty value is -1.
+        const int nOut = L->numOutliers;
+        size_t blockEnd = 0;
+        auto place = [&](size_t bytes) {
+            const size_t at = blockEnd;
+            blockEnd = (blockEnd + bytes + 255) & ~size_t(255);
+            return at;
+        };
+        const size_t oFilm = place(memory != SST_MEM_DEVICE ? P * 12 : 0), oVar = place(wantVar ? P * 8 : 0);
+        const size_t oAlb = place(L->albedo ? P * 12 : 0), oNrm = place(L->albedo ? P * 12 : 0), oOutW = place(P * size_t(nOut) * 4);
+        const size_t clearBytes = blockEnd, oOutIt = place(P * size_t(nOut) * 4);
+        c->layBlock.ensure(std::max<size_t>(256, blockEnd));
+        char* const block = c->layBlock.as<char>();
         float* dFilm = film;
-        if (memory != SST_MEM_DEVICE) {
-            c->film.ensure(P * 12);
-            dFilm = c->film.as<float>();
-            if (resume) CUDA_CHECK(cudaMemcpyAsync(dFilm, film, P * 12, cudaMemcpyHostToDevice, st));
+        if (memory != SST_MEM_DEVICE) dFilm = reinterpret_cast<float*>(block + oFilm);
+        if (resume) {
+            if (memory != SST_MEM_DEVICE) CUDA_CHECK(cudaMemcpyAsync(dFilm, film, P * 12, cudaMemcpyHostToDevice, st));
+        } else {
+            if (memory == SST_MEM_DEVICE) CUDA_CHECK(cudaMemsetAsync(dFilm, 0, P * 12, st));
+            if (clearBytes) CUDA_CHECK(cudaMemsetAsync(block, 0, clearBytes, st));
+            if (nOut > 0) CUDA_CHECK(cudaMemsetAsync(block + oOutIt, 0xFF, P * size_t(nOut) * 4, st));
         }
-        if (!resume) CUDA_CHECK(cudaMemsetAsync(dFilm, 0, P * 12, st));
         std::vector<JobIn> jobs(1);
         jobs[0].s = s;
         jobs[0].p = *p;
@@ -868,20 +909,18 @@ int sst_render_layers(sst_scene* s, const SstPathTracerParams* p, float* film, i
         jobs[0].iterFirst = first;
         jobs[0].iterEnd = std::max(first, S);
         DevLayers& lay = jobs[0].lay;
-        // layer state: read back in when resuming, zero otherwise
-        auto state = [&](DevBuf& b, size_t bytes, const float* src) {
-            b.ensure(bytes);
-            if (resume) CUDA_CHECK(cudaMemcpyAsync(b.p, src, bytes, in, st));
-            else CUDA_CHECK(cudaMemsetAsync(b.p, 0, bytes, st));
-            return b.as<float>();
+        // layer state: read back in when resuming
+        auto state = [&](size_t at, size_t bytes, const void* src) {
+            if (resume) CUDA_CHECK(cudaMemcpyAsync(block + at, src, bytes, in, st));
+            return reinterpret_cast<float*>(block + at);
         };
         if (wantVar) {
-            lay.varMean = state(c->layMean, P * 8, L->varianceState);  // mean plane, then moment plane
+            lay.varMean = state(oVar, P * 8, L->varianceState);  // mean plane, then moment plane
             lay.varMoment = lay.varMean + P;
         }
         if (L->albedo) {
-            lay.aovAlbedo = state(c->layAlb, P * 12, L->albedo);
-            lay.aovNormal = state(c->layNrm, P * 12, L->normal);
+            lay.aovAlbedo = state(oAlb, P * 12, L->albedo);
+            lay.aovNormal = state(oNrm, P * 12, L->normal);
         }
         if (L->reference) {
             lay.ref = toDevice(c, c->layRef, L->reference, P * 3, L->memory);
@@ -903,22 +942,11 @@ int sst_render_layers(sst_scene* s, const SstPathTracerParams* p, float* film, i
             lay.pyr = c->layPyr.as<float>();
             lay.pyrSpp = p->totalSpp;
         }
-        const int nOut = L->numOutliers;
         if (nOut > 0) {
             // OutlierReplayCache: created empty with the frame buffer's first iteration, kept after that
-            const size_t n = P * size_t(nOut);
-            c->layOutW.ensure(n * 4);
-            c->layOutIt.ensure(n * 4);
-            if (resume) {
-                CUDA_CHECK(cudaMemcpyAsync(c->layOutW.p, L->outlierWeight, n * 4, in, st));
-                CUDA_CHECK(cudaMemcpyAsync(c->layOutIt.p, L->outlierIteration, n * 4, in, st));
-            } else {
-                CUDA_CHECK(cudaMemsetAsync(c->layOutW.p, 0, n * 4, st));
-                CUDA_CHECK(cudaMemsetAsync(c->layOutIt.p, 0xFF, n * 4, st));
-            }
             lay.nOut = nOut;
-            lay.outW = c->layOutW.as<float>();
-            lay.outIt = c->layOutIt.as<int>();
+            lay.outW = state(oOutW, P * size_t(nOut) * 4, L->outlierWeight);
+            lay.outIt = reinterpret_cast<int*>(state(oOutIt, P * size_t(nOut) * 4, L->outlierIteration));
         }
         HostPrefault prefault;
         if (memory != SST_MEM_DEVICE) prefault.add(film, P * 12);
@@ -935,14 +963,25 @@ int sst_render_layers(sst_scene* s, const SstPathTracerParams* p, float* film, i
                 prefault.add(L->normal, P * 12);
             }
         }
-        prefault.start();
-        if (first < S) renderJobs(c, jobs, &local);
+        if (first < S) renderJobs(c, jobs, &local, false, nullptr, &prefault);
         prefault.finish();
+        // The block of a small image comes back in one copy into page-locked memory; the copies of its
+        // sections into the caller's arrays below then read that.  Up to 128 KB: a copy into ordinary memory
+        // costs about 12 us however small, and the second pass over the data about 130 us per MB.
+        const bool oneCopy = memory != SST_MEM_DEVICE && L->memory != SST_MEM_DEVICE && blockEnd <= kLayStageBytes;
+        if (oneCopy) {
+            c->layStage.ensure(kLayStageBytes);
+            CUDA_CHECK(cudaMemcpyAsync(c->layStage.p, block, blockEnd, cudaMemcpyDeviceToHost, st));
+        }
+        std::vector<std::pair<void*, std::pair<size_t, size_t>>> fromStage;  // destination, section, bytes
+        auto section = [&](void* dst, size_t at, size_t bytes, cudaMemcpyKind kind) {
+            if (oneCopy) fromStage.push_back({dst, {at, bytes}});
+            else CUDA_CHECK(cudaMemcpyAsync(dst, block + at, bytes, kind, st));
+        };
         if (L->techPyramid) CUDA_CHECK(cudaMemcpyAsync(L->techPyramid, lay.pyr, 2 * 2 * size_t(p->maxDepth) * P * 12, out, st));
         if (nOut > 0) {
-            const size_t n = P * size_t(nOut);
-            CUDA_CHECK(cudaMemcpyAsync(L->outlierWeight, lay.outW, n * 4, out, st));
-            CUDA_CHECK(cudaMemcpyAsync(L->outlierIteration, lay.outIt, n * 4, out, st));
+            section(L->outlierWeight, oOutW, P * size_t(nOut) * 4, out);
+            section(L->outlierIteration, oOutIt, P * size_t(nOut) * 4, out);
         }
         std::vector<double> trim;
         if (lay.errPix) {
@@ -956,7 +995,7 @@ int sst_render_layers(sst_scene* s, const SstPathTracerParams* p, float* film, i
             CUDA_CHECK(cudaMemcpyAsync(trim.data(), c->layTrim.p, size_t(nIt) * 8, cudaMemcpyDeviceToHost, st));
         }
         if (wantVar) {
-            CUDA_CHECK(cudaMemcpyAsync(L->varianceState, lay.varMean, P * 8, out, st));
+            section(L->varianceState, oVar, P * 8, out);
             c->layVar.ensure(P * 4);
             c->laySum.ensure(8);
             CUDA_CHECK(cudaMemsetAsync(c->laySum.p, 0, 8, st));
@@ -973,8 +1012,8 @@ int sst_render_layers(sst_scene* s, const SstPathTracerParams* p, float* film, i
             }
         }
         if (L->albedo) {
-            CUDA_CHECK(cudaMemcpyAsync(L->albedo, lay.aovAlbedo, P * 12, out, st));
-            CUDA_CHECK(cudaMemcpyAsync(L->normal, lay.aovNormal, P * 12, out, st));
+            section(L->albedo, oAlb, P * 12, out);
+            section(L->normal, oNrm, P * 12, out);
         }
         if (L->errors && first < S) {
             std::vector<double> e(2 * size_t(S));
@@ -990,8 +1029,9 @@ int sst_render_layers(sst_scene* s, const SstPathTracerParams* p, float* film, i
             if (L->memory == SST_MEM_DEVICE) CUDA_CHECK(cudaMemcpy(L->errors, res.data(), res.size() * 8, cudaMemcpyHostToDevice));
             else std::copy(res.begin(), res.end(), L->errors);
         }
-        if (memory != SST_MEM_DEVICE) CUDA_CHECK(cudaMemcpyAsync(film, dFilm, P * 12, cudaMemcpyDeviceToHost, st));
+        if (memory != SST_MEM_DEVICE) section(film, oFilm, P * 12, cudaMemcpyDeviceToHost);
         CUDA_CHECK(cudaStreamSynchronize(st));
+        for (auto& x : fromStage) std::memcpy(x.first, c->layStage.as<char>() + x.second.first, x.second.second);
         if (stats) *stats = local;
     });
 }
@@ -1009,8 +1049,7 @@ int sst_render_batch(sst_ctx* ctx, const SstRenderJob* jobs, int32_t numJobs, Ss
         HostPrefault prefault;
         for (int j = 0; j < numJobs; ++j)
             if (jobs[j].memory != SST_MEM_DEVICE) prefault.add(jobs[j].film, size_t(jobs[j].params.width) * jobs[j].params.height * 12);
-        prefault.start();
-        renderJobs(ctx, in, &total);
+        renderJobs(ctx, in, &total, false, nullptr, &prefault);
         prefault.finish();
         auto t1 = std::chrono::steady_clock::now();
         batchFilmsOut(ctx, jobs, numJobs, in);
