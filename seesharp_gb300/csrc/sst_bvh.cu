@@ -722,7 +722,8 @@ void launch_leaf_gather(const int* order, int n, const float4* trivG, const floa
 // remain); leaves are shared unchanged.  Level-synchronous: one launch per level of the 4-wide
 // tree, the frontier holds the level's binary nodes in the order of their 4-wide slots.
 // Node layout (8 float4, 128 bytes): lo.x[4], hi.x[4], lo.y[4], hi.y[4], lo.z[4], hi.z[4],
-// child references[4] (a 4-wide node index or a leaf reference), (number of children, -, -, -).
+// child references[4] (a 4-wide node index or a leaf reference), one unused float4 (a node is one
+// 128-byte line).  Nodes with fewer children have inside-out boxes in the other places.
 // =============================================================================================
 namespace sst {
 namespace {
@@ -813,13 +814,14 @@ __global__ void k_collapse4(const float4* nodes2, const int* frontier, Levels* l
             }
             refs[k] = r;
         } else {
-            for (int a = 0; a < 6; ++a) v[a][k] = 0.0f;
+            // an inside-out box: its near planes lie at +inf and its far ones at -inf for every direction
+            for (int a = 0; a < 6; ++a) v[a][k] = (a & 1) ? -CUDART_INF_F : CUDART_INF_F;
             refs[k] = 0u;
         }
     }
     for (int a = 0; a < 6; ++a) out[a] = make_float4(v[a][0], v[a][1], v[a][2], v[a][3]);
     out[6] = make_float4(__uint_as_float(refs[0]), __uint_as_float(refs[1]), __uint_as_float(refs[2]), __uint_as_float(refs[3]));
-    out[7] = make_float4(__int_as_float(cnt), 0.0f, 0.0f, 0.0f);
+    out[7] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 }
 __global__ void k_collapse_root(int* frontier, Levels* lv) {
     *lv = Levels{{1, 0, 0}, {0, 1, 0}, 0};

@@ -1,5 +1,5 @@
 """Rays that no triangle can meet (an origin that is not finite, a NaN in the direction, a direction of
-length zero) end as misses in every traversal width, beside ordinary rays whose hits they do not change.
+length zero or with infinite components) end as misses in every traversal width, beside ordinary rays whose hits they do not change.
 
 The CPU part evaluates the watertight edge functions (Woop, Benthin, Wald 2013) in numpy's single
 precision for such rays: the distance is never inside any interval, which is what the early end states.
@@ -23,6 +23,8 @@ def _lost_rays():
         d[k] = NAN
         out.append((np.array([0.1, 0.2, 0.3], np.float32), d))
     out.append((np.zeros(3, np.float32), np.zeros(3, np.float32)))
+    for d in ([INF, 0.3, 0.2], [0.1, -INF, 0.2], [INF, INF, 0.2], [-INF, 0.1, INF], [INF, -INF, INF]):
+        out.append((np.array([0.1, 0.2, 0.3], np.float32), np.array(d, np.float32)))
     out.append((np.full(3, NAN), np.full(3, NAN)))
     out.append((np.full(3, INF), np.array([0, 0, 1], np.float32)))
     return out
@@ -73,7 +75,7 @@ def test_lost_rays_miss(width):
         want, blocked = sc.native.trace(rays), sc.native.occluded(rays)
         mixed, at = rays.copy(), []
         for k, (o, d) in enumerate(_lost_rays()):
-            at.append(17 + 211 * k)
+            at.append(17 + 173 * k)
             mixed[at[-1], 0:3], mixed[at[-1], 4:7] = o, d
         got, got_blocked = sc.native.trace(mixed), sc.native.occluded(mixed)
     finally:
