@@ -21,8 +21,7 @@ int sst_forward_batch(sst_ctx* ctx, const SstRenderJob* jobs, int32_t numJobs, S
         CUDA_CHECK(cudaSetDevice(ctx->device));
         ctx->batchSig.clear();
         std::vector<JobIn> in;
-        std::vector<std::unique_ptr<DevBuf>> staged;
-        batchJobs(ctx, jobs, numJobs, in, staged, true);
+        batchJobs(ctx, jobs, numJobs, in, true);
         if ((int)ctx->batchRecord.size() < numJobs) ctx->batchRecord.resize(numJobs);
         for (int j = 0; j < numJobs; ++j) {
             size_t P = size_t(jobs[j].params.width) * jobs[j].params.height;
@@ -59,8 +58,7 @@ int sst_backward_batch(sst_ctx* ctx, const SstRenderJob* jobs, int32_t numJobs, 
         CUDA_CHECK(cudaSetDevice(ctx->device));
         cudaStream_t st = ctx->stream;
         std::vector<JobIn> in;
-        std::vector<std::unique_ptr<DevBuf>> staged;
-        batchJobs(ctx, jobs, numJobs, in, staged, true);
+        batchJobs(ctx, jobs, numJobs, in, true);
         if ((int)ctx->batchDLdI.size() < numJobs) ctx->batchDLdI.resize(numJobs);
         // gradient buffers of each distinct scene, zeroed once
         std::vector<sst_scene*> scenes;

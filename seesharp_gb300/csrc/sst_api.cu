@@ -45,6 +45,17 @@ int sst_create(int32_t device, sst_ctx** out) {
             for (cudaEvent_t* e : {&ws.evShade, &ws.evShadow, &ws.evDone, &ws.evFolded}) CUDA_CHECK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
         }
         CUDA_CHECK(cudaMallocHost(&c->pinnedCount, sizeof(int) * 4));
+        int pools = 0;
+        CUDA_CHECK(cudaDeviceGetAttribute(&pools, cudaDevAttrMemoryPoolsSupported, device));
+        if (pools) {
+            cudaMemPoolProps props{};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = device;
+            CUDA_CHECK(cudaMemPoolCreate(&c->scenePool, &props));
+            uint64_t keep = kScenePoolBytes;
+            CUDA_CHECK(cudaMemPoolSetAttribute(c->scenePool, cudaMemPoolAttrReleaseThreshold, &keep));
+        }
         *out = c.release();
     });
 }
@@ -68,6 +79,7 @@ int sst_destroy(sst_ctx* ctx) {
             if (ws.side) cudaStreamDestroy(ws.side);
             if (ws.run) cudaStreamDestroy(ws.run);
         }
+        if (ctx->scenePool) cudaMemPoolDestroy(ctx->scenePool);
         cudaStreamDestroy(ctx->stream);
         delete ctx;
     });
@@ -76,9 +88,7 @@ int sst_destroy(sst_ctx* ctx) {
 int sst_scene_create(sst_ctx* ctx, sst_scene** out) {
     return guarded([&] {
         if (!ctx || !out) fail(SST_ERR_INVALID_ARGUMENT, "NULL argument");
-        auto s = std::make_unique<sst_scene>();
-        s->ctx = ctx;
-        *out = s.release();
+        *out = new sst_scene(ctx);
     });
 }
 
