@@ -38,6 +38,7 @@ extern "C" {
 
 #define SST_MEM_HOST 0
 #define SST_MEM_DEVICE 1
+#define SST_MEM_HOST_PLANES 2 /* sst_trace_light_paths only: host memory, the vertices' floats and integers apart */
 
 #define SST_BORDER_REPEAT 0 /* ImageTexture.BorderHandling.Repeat (Images/ImageTexture.cs:12-21) */
 #define SST_BORDER_CLAMP 1  /* ImageTexture.BorderHandling.Clamp */
@@ -279,7 +280,8 @@ typedef struct SstPathVertex {
     int32_t fromBackground;
     int32_t reserved;
 } SstPathVertex;
-/* vertices: numPaths * (maxDepth + 1) entries, path i at i * (maxDepth + 1); lengths: numPaths. */
+/* vertices: numPaths * (maxDepth + 1) entries, path i at i * (maxDepth + 1); lengths: numPaths.
+ * With SST_MEM_HOST_PLANES the entries' 16 floats come first, all of them, and then their 6 integers. */
 int sst_trace_light_paths(sst_scene* scene, uint32_t seed, uint32_t iteration, int32_t numPaths, int32_t maxDepth, SstPathVertex* vertices,
                           int32_t* lengths, int32_t memory, SstRenderStats* stats);
 

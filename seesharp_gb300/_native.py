@@ -16,6 +16,7 @@ LIB_PATH = os.path.join(HERE, "libsst.so")
 
 SST_MEM_HOST = 0
 SST_MEM_DEVICE = 1
+SST_MEM_HOST_PLANES = 2  # sst_trace_light_paths: the vertices' floats and integers apart
 SST_NOALLOC_MAX_RAYS = 65536  # rays per sst_occluded_noalloc call
 
 _ERRORS = {
@@ -438,12 +439,14 @@ class SceneHandle:
         """sst_trace_light_paths: (floats (n, maxDepth+1, 16), ints (n, maxDepth+1, 6), lengths (n,),
         stats) in the layout of SstPathVertex."""
         stride = max_depth + 1
-        raw = np.zeros((num_paths, stride, 22), np.float32)
+        n = num_paths * stride
+        # one block, written whole by the call: all floats, then all integers
+        raw = np.empty(22 * n, np.float32)
         lengths = np.zeros(num_paths, np.int32)
         stats = SstRenderStats()
         check(self.lib.sst_trace_light_paths(self.handle, seed & 0xFFFFFFFF, iteration & 0xFFFFFFFF, int(num_paths), int(max_depth), ptr(raw),
-                                              ptr(lengths), SST_MEM_HOST, ctypes.byref(stats)))
-        return raw[..., :16].copy(), raw[..., 16:].copy().view(np.int32), lengths, stats
+                                              ptr(lengths), SST_MEM_HOST_PLANES, ctypes.byref(stats)))
+        return raw[:16 * n].reshape(num_paths, stride, 16), raw[16 * n:].view(np.int32).reshape(num_paths, stride, 6), lengths, stats
 
     def update_texture(self, tex_id, data):
         d = np.ascontiguousarray(data, np.float32)

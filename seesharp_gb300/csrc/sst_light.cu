@@ -222,7 +222,8 @@ SST_D bool sampleFull(const DevScene& sc, const DevMaterial& m, const Lp& lp, fl
     return true;
 }
 
-SST_D void putVertex(SstPathVertexDev* out, const Surf& s, bool surface, int mesh, int face, float pdfFrom, float pdfRev, float3 weight,
+// Writes vertex `at` (path * (maxDepth + 1) + its place on the path).
+SST_D void putVertex(const LightVerts& verts, size_t at, const Surf& s, bool surface, int mesh, int face, float pdfFrom, float pdfRev, float3 weight,
                      float rough, int depth, int path, bool fromBg) {
     SstPathVertexDev v;
     v.p[0] = s.pos.x; v.p[1] = s.pos.y; v.p[2] = s.pos.z;
@@ -232,7 +233,10 @@ SST_D void putVertex(SstPathVertexDev* out, const Surf& s, bool surface, int mes
     v.p[12] = weight.x; v.p[13] = weight.y; v.p[14] = weight.z;
     v.p[15] = rough;
     v.q[0] = surface ? mesh : -1; v.q[1] = surface ? face : -1; v.q[2] = depth; v.q[3] = path; v.q[4] = fromBg ? 1 : 0; v.q[5] = 0;
-    *out = v;
+    float* p = verts.p + at * verts.pStride;
+    int* q = verts.q + at * verts.qStride;
+    for (int k = 0; k < 16; ++k) p[k] = v.p[k];
+    for (int k = 0; k < 6; ++k) q[k] = v.q[k];
 }
 
 }  // namespace
@@ -242,14 +246,14 @@ SST_D void putVertex(SstPathVertexDev* out, const Surf& s, bool surface, int mes
 // TraceBackgroundPath, :151-241; DiffuseEmitter.SampleRay, GlossyEmitter.SampleRay,
 // EnvironmentMap.SampleRay)
 // ---------------------------------------------------------------------------------------------
-__global__ void k_light_start(const DevJob* jobs, LightParams P, LightPathBuf A, int* qCount, SstPathVertexDev* verts, int* lengths) {
+__global__ void k_light_start(const DevJob* jobs, LightParams P, LightPathBuf A, int* qCount, LightVerts verts, int* lengths) {
     int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= P.numPaths) return;
     const DevScene& sc = jobs[0].sc;
     Rng rng{hashSeed(P.seed, (uint32_t)idx, P.iter)};
     const int nEm = sc.nEmitters;
     const int stride = P.maxDepth + 1;
-    SstPathVertexDev* out = verts + (size_t)idx * stride;
+    const size_t out = (size_t)idx * stride;
     float bgProb = sc.hasEnv ? 1.0f / (1.0f + (float)nEm) : 0.0f;
     bool background = false;
     float prob;
@@ -293,7 +297,7 @@ __global__ void k_light_start(const DevJob* jobs, LightParams P, LightPathBuf A,
         float3 dir = local.z * s0.sn + local.x * t + local.y * b;
         float pdf = lpdf * posPdf * prob;
         if (pdf == 0.0f || isBlack(weight)) { lengths[idx] = 0; return; }
-        putVertex(out, s0, true, em.mesh, em.face, 0.0f, 0.0f, mk(0, 0, 0), 0.0f, 0, idx, false);
+        putVertex(verts, out, s0, true, em.mesh, em.face, 0.0f, 0.0f, mk(0, 0, 0), 0.0f, 0, idx, false);
         lengths[idx] = 1;
         if (1 >= P.maxDepth) return;  // RandomWalk.ContinueWalk: while (depth < maxDepth)
         ro = offsetPoint(s0.pos, s0.n, s0.eps, dir);
@@ -320,7 +324,7 @@ __global__ void k_light_start(const DevJob* jobs, LightParams P, LightPathBuf A,
         weight = weight / prob;
         if (pdf == 0.0f || isBlack(weight)) { lengths[idx] = 0; return; }
         s0.pos = pos;
-        putVertex(out, s0, false, -1, -1, 0.0f, 0.0f, mk(0, 0, 0), 0.0f, 0, idx, true);
+        putVertex(verts, out, s0, false, -1, -1, 0.0f, 0.0f, mk(0, 0, 0), 0.0f, 0, idx, true);
         lengths[idx] = 1;
         ro = pos;
         rd = -dsd;
@@ -345,7 +349,7 @@ __global__ void k_light_start(const DevJob* jobs, LightParams P, LightPathBuf A,
 // background path's first hit, RandomWalk.ContinueWalk :145-216 otherwise)
 // ---------------------------------------------------------------------------------------------
 __global__ void k_light_walk(const DevJob* jobs, LightParams P, LightPathBuf A, LightPathBuf B, const float4* hits, const int* nIn, int* nOut,
-                             SstPathVertexDev* verts, int* lengths) {
+                             LightVerts verts, int* lengths) {
     const int n = *nIn;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if ((int)(blockIdx.x * blockDim.x) >= n) return;
@@ -370,7 +374,7 @@ __global__ void k_light_walk(const DevJob* jobs, LightParams P, LightPathBuf A, 
         float4 h = hits[i];
         int ti = __float_as_int(h.w);
         const int stride = P.maxDepth + 1;
-        SstPathVertexDev* out = verts + (size_t)path * stride;
+        const size_t out = (size_t)path * stride;
         if (ti >= 0) {
             float3 rdir = f3(A.rd[i]);
             Surf s;
@@ -399,7 +403,7 @@ __global__ void k_light_walk(const DevJob* jobs, LightParams P, LightPathBuf A, 
                 bool ok = sampleFull(sc, m, lp, diffBase, c, true, uc, u1, u2, dirW, bp, bpr, bw);
                 if (!ok) { bp = 0.0f; bpr = 0.0f; bw = mk(0, 0, 0); }
                 approx = approx * bw;
-                putVertex(out + len, s, true, mesh, face, pdfDir, nextRev, prefix, rough, 1, (int)path, fromBg);
+                putVertex(verts, out + len, s, true, mesh, face, pdfDir, nextRev, prefix, rough, 1, (int)path, fromBg);
                 lengths[path] = len + 1;
                 nextRev = bpr;
                 if (P.maxDepth > 1 && bp != 0.0f && !isBlack(bw)) {
@@ -415,7 +419,7 @@ __global__ void k_light_walk(const DevJob* jobs, LightParams P, LightPathBuf A, 
             } else {
                 float pdfFrom = pdfDir * areaToSolidAngle(prevPos, s.pos, s.n);
                 if (pdfFrom != 0.0f) {
-                    putVertex(out + len, s, true, mesh, face, pdfFrom, nextRev, prefix, rough, depth, (int)path, fromBg);
+                    putVertex(verts, out + len, s, true, mesh, face, pdfFrom, nextRev, prefix, rough, depth, (int)path, fromBg);
                     lengths[path] = len + 1;
                     if (depth + 1 < P.maxDepth) {
                         float surv = depth > 4 ? clampf(avg3(approx), 0.05f, 0.95f) : 1.0f;
@@ -466,14 +470,14 @@ __global__ void k_light_walk(const DevJob* jobs, LightParams P, LightPathBuf A, 
     B.rd[j] = make_float4(nrd.x, nrd.y, nrd.z, CUDART_INF_F);
 }
 
-void launch_light_start(const DevJob* jobs, const LightParams& P, const LightPathBuf& A, int* qCount, SstPathVertexDev* verts, int* lengths,
+void launch_light_start(const DevJob* jobs, const LightParams& P, const LightPathBuf& A, int* qCount, const LightVerts& verts, int* lengths,
                         cudaStream_t s) {
     if (P.numPaths <= 0) return;
     k_light_start<<<(P.numPaths + 127) / 128, 128, 0, s>>>(jobs, P, A, qCount, verts, lengths);
 }
 
 void launch_light_walk(const DevJob* jobs, const LightParams& P, const LightPathBuf& A, const LightPathBuf& B, const float4* hits, const int* nIn,
-                       int* nOut, SstPathVertexDev* verts, int* lengths, int maxItems, cudaStream_t s) {
+                       int* nOut, const LightVerts& verts, int* lengths, int maxItems, cudaStream_t s) {
     if (maxItems <= 0) return;
     k_light_walk<<<(maxItems + 127) / 128, 128, 0, s>>>(jobs, P, A, B, hits, nIn, nOut, verts, lengths);
 }

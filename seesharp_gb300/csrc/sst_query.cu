@@ -122,15 +122,23 @@ int sst_trace_light_paths(sst_scene* s, uint32_t seed, uint32_t iteration, int32
         const size_t n = size_t(numPaths), stride = size_t(maxDepth) + 1;
         LightPathBuf A = bindLight(c->lightA, n), B = bindLight(c->lightB, n);
         c->lightHits.ensure(n * 16);
-        SstPathVertexDev* dv = reinterpret_cast<SstPathVertexDev*>(vertices);
+        const size_t words = n * stride * (sizeof(SstPathVertexDev) / 4);
+        float* dv = reinterpret_cast<float*>(vertices);
         int* dl = lengths;
         if (memory != SST_MEM_DEVICE) {
-            c->lightVerts.ensure(n * stride * sizeof(SstPathVertexDev));
+            c->lightVerts.ensure(words * 4);
             c->lightLengths.ensure(n * 4);
-            dv = c->lightVerts.as<SstPathVertexDev>();
+            dv = c->lightVerts.as<float>();
             dl = c->lightLengths.as<int>();
         }
-        CUDA_CHECK(cudaMemsetAsync(dv, 0, n * stride * sizeof(SstPathVertexDev), st));
+        const LightVerts lv = memory == SST_MEM_HOST_PLANES ? LightVerts{dv, reinterpret_cast<int*>(dv + n * stride * 16), 16, 6}
+                                                            : LightVerts{dv, reinterpret_cast<int*>(dv + 16), 22, 22};
+        CUDA_CHECK(cudaMemsetAsync(dv, 0, words * 4, st));
+        HostPrefault prefault;
+        if (memory != SST_MEM_DEVICE) {
+            prefault.add(vertices, words * 4);
+            prefault.add(lengths, n * 4);
+        }
         c->lightCnt.ensure(sizeof(int) * 2 * (size_t(maxDepth) + 3));
         int* cnt = c->lightCnt.as<int>();
         CUDA_CHECK(cudaMemsetAsync(cnt, 0, sizeof(int) * 2 * (size_t(maxDepth) + 3), st));
@@ -140,8 +148,9 @@ int sst_trace_light_paths(sst_scene* s, uint32_t seed, uint32_t iteration, int32
         const DevJob* job = s->queryJob.as<DevJob>();
         LightParams P{numPaths, maxDepth, seed, iteration};
         CUDA_CHECK(cudaEventRecord(c->ev0, st));
-        launch_light_start(job, P, A, cnt, dv, dl, st);
+        launch_light_start(job, P, A, cnt, lv, dl, st);
         CUDA_CHECK(cudaGetLastError());
+        prefault.start();
         int items = 0;
         CUDA_CHECK(cudaMemcpyAsync(&items, cnt, sizeof(int), cudaMemcpyDeviceToHost, st));
         CUDA_CHECK(cudaStreamSynchronize(st));
@@ -151,15 +160,16 @@ int sst_trace_light_paths(sst_scene* s, uint32_t seed, uint32_t iteration, int32
             int* qOut = cnt + d + 1;
             int* work = cnt + (maxDepth + 2) + d;
             launch_trace_closest(tt, job, nullptr, A.ro, A.rd, qIn, work, c->lightHits.as<float4>(), c->stats.as<DevStats>(), st);
-            launch_light_walk(job, P, A, B, c->lightHits.as<float4>(), qIn, qOut, dv, dl, items, st);
+            launch_light_walk(job, P, A, B, c->lightHits.as<float4>(), qIn, qOut, lv, dl, items, st);
             CUDA_CHECK(cudaGetLastError());
             std::swap(A, B);
             CUDA_CHECK(cudaMemcpyAsync(&items, qOut, sizeof(int), cudaMemcpyDeviceToHost, st));
             CUDA_CHECK(cudaStreamSynchronize(st));
         }
         CUDA_CHECK(cudaEventRecord(c->ev1, st));
+        prefault.finish();
         if (memory != SST_MEM_DEVICE) {
-            CUDA_CHECK(cudaMemcpyAsync(vertices, dv, n * stride * sizeof(SstPathVertexDev), cudaMemcpyDeviceToHost, st));
+            CUDA_CHECK(cudaMemcpyAsync(vertices, dv, words * 4, cudaMemcpyDeviceToHost, st));
             CUDA_CHECK(cudaMemcpyAsync(lengths, dl, n * 4, cudaMemcpyDeviceToHost, st));
         }
         DevStats hs;

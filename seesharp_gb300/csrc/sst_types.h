@@ -136,6 +136,13 @@ struct SstPathVertexDev {  // the layout of SstPathVertex
     float p[16];
     int q[6];
 };
+// Where the light paths' vertices go: one array of SstPathVertex records (strides of 22 words), or their
+// 16 floats and their 6 integers in an array each.
+struct LightVerts {
+    float* p;
+    int* q;
+    int pStride, qStride;
+};
 
 // Frame-buffer layers of a job (all NULL unless requested).
 struct DevLayers {
