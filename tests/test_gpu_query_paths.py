@@ -45,3 +45,21 @@ def test_results_do_not_depend_on_the_route(scene, n):
         _native.check(sh.lib.sst_trace(sh.handle, p, n, ctypes.c_void_p(out.data_ptr()), _native.SST_MEM_DEVICE))
         _native.check(sh.lib.sst_occluded(sh.handle, p, n, ctypes.c_void_p(oc.data_ptr()), _native.SST_MEM_DEVICE))
         assert np.array_equal(out.cpu().numpy().view(np.uint32), hits.view(np.uint32)) and np.array_equal(oc.cpu().numpy(), occ)
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 255, 257, 4099])
+@pytest.mark.parametrize("shift", [0, 1, 2, 3])  # floats from a 16-byte boundary
+def test_device_hits_on_any_boundary(scene, n, shift):
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(n)
+    rays = np.zeros((n, 8), np.float32)
+    rays[:, 0:3], rays[:, 4:7], rays[:, 7] = rng.uniform(0, 20, (n, 3)), rng.standard_normal((n, 3)), np.inf
+    sh = scene.native
+    hits = sh.trace(rays)
+    d = torch.from_numpy(rays).cuda()
+    out = torch.full((12 * n + 8,), 7.0, device="cuda")
+    torch.cuda.synchronize()
+    _native.check(sh.lib.sst_trace(sh.handle, ctypes.c_void_p(d.data_ptr()), n, ctypes.c_void_p(out.data_ptr() + 4 * shift), _native.SST_MEM_DEVICE))
+    o = out.cpu().numpy()
+    assert np.array_equal(o[shift:shift + 12 * n].view(np.uint32), hits.reshape(-1).view(np.uint32))
+    assert np.all(o[:shift] == 7.0) and np.all(o[shift + 12 * n:] == 7.0)
