@@ -119,6 +119,12 @@ static void checkTex(sst_scene* s, int tex, int wantCh) {
     (void)wantCh;
 }
 
+// A committed scene's material updates are copies without a wait, and adding a material may move the array
+// that they read (a system whose devices read pageable memory directly need not stage them).
+static void settleUpdates(sst_scene* s) {
+    if (s->mats.p) CUDA_CHECK(cudaStreamSynchronize(s->ctx->stream));
+}
+
 int sst_scene_add_material_diffuse(sst_scene* s, const float base[3], int32_t tex, int32_t transmitter, int32_t* out) {
     return guarded([&] {
         if (!s || !base || !out) fail(SST_ERR_INVALID_ARGUMENT, "NULL argument");
@@ -131,6 +137,7 @@ int sst_scene_add_material_diffuse(sst_scene* s, const float base[3], int32_t te
         for (int k = 0; k < 3; ++k) m.base[k] = base[k];
         m.rough = 1.0f;
         m.ior = 1.0f;
+        settleUpdates(s);
         s->materials.push_back(m);
         s->committed = false;
         *out = int(s->materials.size()) - 1;
@@ -157,7 +164,9 @@ static DevMaterial genericFrom(sst_scene* s, const SstGenericMaterial* p) {
 int sst_scene_add_material_generic(sst_scene* s, const SstGenericMaterial* p, int32_t* out) {
     return guarded([&] {
         if (!s || !p || !out) fail(SST_ERR_INVALID_ARGUMENT, "NULL argument");
-        s->materials.push_back(genericFrom(s, p));
+        const DevMaterial m = genericFrom(s, p);
+        settleUpdates(s);
+        s->materials.push_back(m);
         s->committed = false;
         *out = int(s->materials.size()) - 1;
     });
@@ -169,9 +178,9 @@ int sst_scene_update_material_generic(sst_scene* s, int32_t material, const SstG
             fail(SST_ERR_INVALID_ARGUMENT, "invalid generic material");
         s->materials[material] = genericFrom(s, p);
         if (s->committed) {
-            // the few bytes are taken from the host before the copy returns, and everything that reads
-            // them is ordered after it on the context's stream (a wait per material took 4 of the 38 ms
-            // of an optimisation step over 300 roughness values)
+            // the source stays in the scene, and everything that reads the copy is ordered after it on the
+            // context's stream (a wait per material took 4 of the 38 ms of an optimisation step over 300
+            // roughness values)
             CUDA_CHECK(cudaMemcpyAsync(s->mats.as<DevMaterial>() + material, &s->materials[material], sizeof(DevMaterial), cudaMemcpyHostToDevice,
                                        s->ctx->stream));
         }

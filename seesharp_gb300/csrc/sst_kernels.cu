@@ -563,7 +563,7 @@ SST_D Ctx ctxFromPoint(const float* p, float3 outW) {
 // traversal record (t, u, v, leaf triangle) expanded with the triangle's mesh, face, position, face
 // normal and error offset (Geometry/Mesh.cs:50-60), one thread per ray.  A warp's 32 records go through
 // shared memory: written field by field they are twelve stores with a stride of 48 bytes, each a
-// partial write to 32 sectors (58 us for 2^20 random rays, 617 us the whole query; as
+// partial write to 32 sectors (58 us for a million random rays, 617 us the whole query; as
 // whole rows 580 us).  Caller's arrays need not be aligned to 16 bytes: those are written by the word.
 __global__ void __launch_bounds__(256) k_hit_expand(DevScene sc, const float4* __restrict__ hits, int n, SstHitDev* out) {
     __shared__ float4 rows[8][3 * 32];
