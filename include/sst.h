@@ -201,7 +201,8 @@ typedef struct SstTuning {
                                  is built for: 8 (64 registers; the default), 10, 12 or 14 (48, 40 or 32
                                  registers: more warps, more spilling; one shadow ray per technique only) */
     int32_t shadeOrder;       /* 1 (the default): each bounce's paths are shaded surface hits first, misses and
-                                 finished paths after them; 0: in queue order */
+                                 finished paths after them (forward waves of up to 65536 paths in queue order
+                                 all the same); 0: in queue order */
     int32_t shadeSplit;       /* 1 (the default): forward renders with GenericMaterials and one shadow ray per
                                  technique shade each bounce with two kernels (hit, emitter MIS, Russian roulette
                                  and next-event estimation; then BSDF sampling and the queue compaction), built for

@@ -467,8 +467,6 @@ __global__ void __launch_bounds__(kPartThreads) k_partition(const uint32_t* __re
 // 32-bit additions of warp sums, whose rounding depends on which paths share a warp.  With the order
 // above the emitter gradients of the differentiable Cornell box (512^2, 32 spp) moved by a relative
 // 3e-4, 20 times what they vary by from run to run, so the replay keeps the order they always had.
-// Also for waves of up to 2^16 paths, whose at most 2 x 2048 additions are no bound and whose few blocks
-// of the kernel above would take longer than many small ones (160 x 90 preview: 2% faster with this).
 __global__ void __launch_bounds__(256) k_partition_warp(const uint32_t* __restrict__ depth, const float4* __restrict__ hits, const int* nIn, int* order,
                                                          int* counts) {
     const int n = *nIn;
@@ -491,7 +489,7 @@ __global__ void __launch_bounds__(256) k_partition_warp(const uint32_t* __restri
 }
 
 void launch_partition(bool replay, const uint32_t* depth, const float4* hits, const int* nIn, int* order, int* counts, int maxItems, cudaStream_t s) {
-    if (replay || maxItems <= (1 << 16)) {
+    if (replay) {
         if (maxItems > 0) k_partition_warp<<<(maxItems + 255) / 256, 256, 0, s>>>(depth, hits, nIn, order, counts);
         return;
     }

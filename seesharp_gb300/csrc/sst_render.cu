@@ -122,6 +122,12 @@ static void planWaves(std::vector<JobIn>& jobs, int cap, bool iterationPerWave, 
     (void)waveIterEnds;
 }
 
+// Waves of up to this many paths are shaded in queue order: they leave most of the GPU idle, so the shade
+// launch lasts as long as its slowest warp in either order, and the order is one more launch per bounce.
+// With the order and without it: Cornell box of 160 x 90, 1 sample, 370 and 346 us, of 256 x 192 439 and
+// 412, sphere field of 256 x 192 858 and 849; above the line the sphere field loses (512 x 512: 1423 and
+// 1446).  The replay keeps the order at every size (its sums depend on it, k_partition_warp).
+constexpr int kOrderItems = 1 << 16;
 constexpr size_t kGraphWaves = 8;  // waves from which several sets replay captured graphs
 
 // Renders the jobs' iterations [iterFirst, iterEnd) into their device films.
@@ -293,6 +299,7 @@ void renderJobs(sst_ctx* c, std::vector<JobIn>& jobs, SstRenderStats* out, bool 
     };
     long long launches = 0;  // kernels issued (in graph mode: the nodes of one wave)
     auto issueWave = [&](int set, cudaStream_t rs, int items, bool allowEarlyExit, bool fold, int* camWave) {
+        const bool order = c->shadeOrder && (replay || items > kOrderItems);
         const WaveBuffers& wb = ws[set].wb;
         WaveStore& sk = c->store[set];
         const DevJob* dj = setJobs[set];
@@ -316,7 +323,7 @@ void renderJobs(sst_ctx* c, std::vector<JobIn>& jobs, SstRenderStats* out, bool 
                 KTimer kt(c, 2);
                 PathBuf Ao = A;
                 if (split) Ao.rec = sk.rec.as<float4>();
-                if (c->shadeOrder) {
+                if (order) {
                     launch_partition(replay, A.depth, wb.hits, cnt + kCntQueue + d, wb.order, cnt + kCntPart + 2 * d, maxItems, rs);
                     Ao.order = wb.order;
                 }
@@ -362,7 +369,7 @@ void renderJobs(sst_ctx* c, std::vector<JobIn>& jobs, SstRenderStats* out, bool 
                 launch_trace_shadow(traceRun, dj, wb.shJob, wb.shRo, wb.shRd, wb.shTgt, cnt + kCntShadow + d, cnt + kCntWork + 2 * d + 1, curNee, dstats, ss);
                 if (overlap) CUDA_CHECK(cudaEventRecord(sk.evShadow, sk.side));
             }
-            launches += (c->shadeOrder ? 4 : 3) + (split ? 1 : 0);  // closest hit, shade order, shade (one or two), shadow rays
+            launches += (order ? 4 : 3) + (split ? 1 : 0);  // closest hit, shade order, shade (one or two), shadow rays
             std::swap(A, B);
             if (allowEarlyExit && d >= 6 && d < maxDepth) {
                 // stop early once the queue is empty (long MaxDepth with Russian roulette)
