@@ -128,7 +128,7 @@ static void planWaves(std::vector<JobIn>& jobs, int cap, bool iterationPerWave, 
 // 412, sphere field of 256 x 192 858 and 849; above the line the sphere field loses (512 x 512: 1423 and
 // 1446).  The replay keeps the order at every size (its sums depend on it, k_partition_warp).
 constexpr int kOrderItems = 1 << 16;
-constexpr size_t kGraphWaves = 8;  // waves from which several sets replay captured graphs
+constexpr size_t kGraphWaves = 8;  // waves from which several sets of a forward pass replay captured graphs
 
 // Renders the jobs' iterations [iterFirst, iterEnd) into their device films.
 // paths: instead of the jobs' iteration ranges, render exactly these single-path chunks (one
@@ -400,7 +400,10 @@ void renderJobs(sst_ctx* c, std::vector<JobIn>& jobs, SstRenderStats* out, bool 
         // on a set's wave is captured once and replayed.  Capturing, instantiating and destroying the
         // graphs takes about 0.5 ms in which the GPU has nothing to do, launching a wave kernel by kernel
         // about 0.1 ms beside a running one: 4 waves (509 x 383, 32 samples) 7.93 ms with graphs, 7.73
-        // without; 5 waves (40 small jobs) 7.57 against 7.38 ms; 32 waves the same either way.
+        // without; 5 waves (40 small jobs) 7.57 against 7.38 ms; 32 waves the same either way.  The replay
+        // keeps the graphs: launched one by one its waves meet differently, and the 32-bit gradient sums round
+        // by the order of their additions (512 x 512, 32 samples, radiance gradients against
+        // the mean of 8 runs with graphs: those 1e-5 apart, without 3e-5, and 3e-4 in one run of eight).
         // the graphs and their executables, released on every way out
         struct Graphs {
             cudaGraph_t g[kMaxWaveSets] = {};
@@ -412,7 +415,7 @@ void renderJobs(sst_ctx* c, std::vector<JobIn>& jobs, SstRenderStats* out, bool 
                 }
             }
         } gr;
-        const bool graphs = waves.size() >= kGraphWaves;
+        const bool graphs = replay || waves.size() >= kGraphWaves;
         long long perWave = 0;
         for (int k = 0; graphs && k < nSets; ++k) {
             cudaStream_t rs = c->store[k].run;
