@@ -72,6 +72,13 @@ struct TraceResult {
     int tri;  // leaf-ordered triangle, -1 for a miss
 };
 
+// The far bound of the wide box tests: the closest hit so far with room for the rounding of box and
+// triangle distances, and never so large that the room makes it infinite.  A child whose planes all
+// overflow to +inf (a short direction among large coordinates) then fails the test, as no triangle has
+// an infinite distance, and the entry distance of every child that passes is finite: the 4-wide node's
+// pushes tell the hit children from the others by that.
+SST_D float farBound(float t) { return fminf(t * 1.0000004f, 3.402822e38f); }
+
 struct Bvh {
     const float4* nodes;
     const float4* triv;
@@ -316,7 +323,7 @@ SST_D bool trav4Run(Trav4& s, int* sstack, int* lstack, int* errFlags, int pause
             const float4 nx = __ldg(nd + ox), fx = __ldg(nd + 1 - ox), ny = __ldg(nd + 2 + oy), fy = __ldg(nd + 3 - oy);
             const float4 nz = __ldg(nd + 4 + oz), fz = __ldg(nd + 5 - oz);
             const float4 rf = __ldg(nd + 6);
-            const float hitT = s.r.t * 1.0000004f;  // conservative far bound (box/triangle rounding)
+            const float hitT = farBound(s.r.t);
             float key[4];
             uint32_t cr[4];
             const float* RF = &rf.x;
@@ -417,7 +424,7 @@ SST_D uint32_t visit8(const Trav8& s, uint32_t node) {
     const float4* nd = s.bvh.nodes8 + 15 * (size_t)node;
     const int ox = (int)(s.oct & 1u), oy = (int)((s.oct >> 1) & 1u), oz = (int)((s.oct >> 2) & 1u);
     const uint32_t valid = __float_as_uint(__ldg(&nd[14].x)) & 0xFFu;
-    const float hitT = s.r.t * 1.0000004f;  // conservative far bound (box/triangle rounding)
+    const float hitT = farBound(s.r.t);
     uint32_t hm = 0;
     // two halves of four children (24 box floats live at a time); near planes: lo for a positive
     // direction component, hi for a negative one
