@@ -87,39 +87,51 @@ struct Bvh {
 SST_D Bvh bvhOf(const DevScene& sc) { return Bvh{sc.nodes, sc.triv, sc.nNodes}; }
 
 // Slab offsets of a ray: a plane p lies at t = p * inv + oi when it is the near one of its axis and at
-// p * inv + of when it is the far one.  oi = of = -origin * inv, but on an axis whose direction component
-// is zero (or so small that p * inv may overflow, or NaN) these products are infinite and the slabs NaN.
-// A NaN slab is ignored by the box tests, so such a ray was culled on its other axes alone, and a lane
-// with two such axes (a cosine-distributed direction with u2 = 1 over a horizontal floor) walked most
+// p * inv + of when it is the far one.  oi = of = -origin * inv, and with a finite oi the fused
+// multiply-add gives every plane's distance, or an infinity on the right side of all of them.  On an axis
+// whose direction component is zero (or too small against the origin) oi is infinite or NaN and the slabs
+// mean nothing.  Ignored, as NaN slabs are, they left such a ray to be culled on its other axes alone, and
+// a lane with two such axes (a cosine-distributed direction with u2 = 1 over a horizontal floor) walked most
 // of the tree while the rest of the GPU idled: on the 1M-triangle scene one path out of 67 million took
 // 300 to 800 ms of a render of 230 ms otherwise, a camera ray with one zero component 2.8 ms.
-// There inv is a power of two, so that p * inv + oi is (p - origin) * inv with one rounding: its sign
-// is exact.  The near plane is passed where it does not lie beyond the origin; the far plane is pushed
-// out by more than any distance, so that an origin exactly on it is inside as well (two triangles that
-// share an edge in the ray's plane keep it watertight).  Every box that holds a triangle such a ray can
-// meet passes, and every other ray's arithmetic is unchanged.
-SST_D void axisSlab(float o, float& inv, float& oi, float& of) {
-    oi = of = -o * inv;
-    if (!(fabsf(inv) < 1e30f)) {
-        inv = copysignf(1.2676506e30f, inv);  // 2^100
-        oi = -o * inv;
-        of = oi + fmaxf(fabsf(oi) * 1e-7f, 1e20f);
-    }
+// axisSlab gives that axis a finite inverse, a power of two, so that p * inv - o * inv is (p - o) * inv with
+// one rounding: its sign is exact.  The near plane is pulled in and the far plane pushed out by `push`: by
+// twice `reach`, which no distance to a box of the scene exceeds, so that they pass whenever the ray can
+// lie inside the slab; by what the component d moves the ray within that reach; and by two ulp of o * inv,
+// so that an origin exactly on a plane is inside (two triangles that share an edge in the ray's plane keep
+// it watertight).  Every box that holds a triangle the ray can meet passes, for directions of any length
+// (up to distances of 2.9e38, where push ends: with finite offsets an empty child's planes stay infinite).
+// Every other axis keeps the plain arithmetic, whatever the size of its component: a component is small
+// only against the others, as directions need not have unit length.
+SST_D void axisSlab(float o, float d, float reach, float& inv, float& oi, float& of) {
+    if (fabsf(oi) < CUDART_INF_F) return;
+    inv = copysignf(1.2676506e30f, inv);  // 2^100
+    const float at = -o * inv;
+    const float push = fminf(reach * (2.0f + fabsf(d * inv)) + fabsf(at) * 2.4e-7f, 2.9e38f);
+    oi = at - push;
+    of = at + push;
 }
-SST_D void raySlabs(float3 org, float3 dir, float3& inv, float3& oi, float3& of) {
+SST_D void raySlabs(const DevScene& sc, float3 org, float3 dir, float3& inv, float3& oi, float3& of) {
     inv = mk(1.0f / dir.x, 1.0f / dir.y, 1.0f / dir.z);
-    axisSlab(org.x, inv.x, oi.x, of.x);
-    axisSlab(org.y, inv.y, oi.y, of.y);
-    axisSlab(org.z, inv.z, oi.z, of.z);
+    oi = of = mk(-org.x * inv.x, -org.y * inv.y, -org.z * inv.z);
+    if (!(fabsf(oi.x) < CUDART_INF_F && fabsf(oi.y) < CUDART_INF_F && fabsf(oi.z) < CUDART_INF_F)) {
+        const float3 c = sc.sceneCenter;
+        const float far = fmaxf(fabsf(c.x), fmaxf(fabsf(c.y), fabsf(c.z))) + sc.sceneRadius + fmaxf(fabsf(org.x), fmaxf(fabsf(org.y), fabsf(org.z)));
+        const float reach = far * fminf(fabsf(inv.x), fminf(fabsf(inv.y), fabsf(inv.z)));
+        axisSlab(org.x, dir.x, reach, inv.x, oi.x, of.x);
+        axisSlab(org.y, dir.y, reach, inv.y, oi.y, of.y);
+        axisSlab(org.z, dir.z, reach, inv.z, oi.z, of.z);
+    }
 }
 // An origin that is not finite: the edge functions or the distance of every triangle are NaN, so the
 // ray misses, and its slabs could not cull anything.
 SST_D bool originLost(float3 o) { return !(fabsf(o.x) < CUDART_INF_F && fabsf(o.y) < CUDART_INF_F && fabsf(o.z) < CUDART_INF_F); }
 
-// A direction of length zero, with a NaN, or with two infinite components: every edge function is NaN and
-// the ray misses.  (Three infinite components would also make the planes of an empty child NaN, the only
-// ones that let a ray into it.)
-SST_D bool noShear(const RayPre& p) { return isnan(p.Sx) || isnan(p.Sy); }
+// A direction without a length in single precision: zero or too short for a finite inverse of its largest
+// component, a NaN, or two infinite components.  The edge functions or the distances of every triangle are
+// NaN or infinite and the ray misses, while its slabs could not cull anything.  (Three infinite components
+// would also make the planes of an empty child NaN, the only ones that let a ray into it.)
+SST_D bool noShear(const RayPre& p) { return isnan(p.Sx) || isnan(p.Sy) || !(fabsf(p.Sz) < CUDART_INF_F); }
 
 // The global id of the closest triangle so far, for a tie in t (no triangle yet loses any tie).  Read
 // back from the triangle record: ties are rare, and the register pays for the second slab offset.
@@ -129,13 +141,15 @@ SST_D int bestId(const float4* triv, int tri) { return tri >= 0 ? __float_as_int
 // sstack: this block's shared stack, SSTACK entries per thread, entry k of thread `tid` at
 // k * BLOCK + tid (consecutive threads in consecutive banks).
 template <bool ANY, int BLOCK, int SSTACK>
-SST_D TraceResult traverse(const Bvh sc, float3 org, float3 dir, float tmin, float tmax, int* sstack, int* errFlags) {
+SST_D TraceResult traverse(const DevScene& scene, float3 org, float3 dir, float tmin, float tmax, int* sstack, int* errFlags) {
+    const Bvh sc = bvhOf(scene);
     TraceResult r{tmax, 0.f, 0.f, -1};
     if (sc.nNodes == 0 || !(tmax > tmin) || originLost(org)) return r;
     int bestGid = 0x7FFFFFFF;
     RayPre pre = rayPre(dir);
+    if (noShear(pre)) return r;
     float3 inv, oi, of;
-    raySlabs(org, dir, inv, oi, of);
+    raySlabs(scene, org, dir, inv, oi, of);
     const bool mx = inv.x < 0.0f, my = inv.y < 0.0f, mz = inv.z < 0.0f;  // hi is the near plane
     int lstack[kMaxStack - SSTACK];
     int sp = 0;
@@ -285,11 +299,12 @@ struct Trav4 {
     bool done;
 };
 
-SST_D void trav4Begin(Trav4& s, const Bvh4 bvh, float3 org, float3 dir, float tmin, float tmax) {
+SST_D void trav4Begin(Trav4& s, const DevScene& sc, float3 org, float3 dir, float tmin, float tmax) {
+    const Bvh4 bvh = bvh4Of(sc);
     s.bvh = bvh;
     s.org = org;
     s.pre = rayPre(dir);
-    raySlabs(org, dir, s.inv, s.oi, s.of);
+    raySlabs(sc, org, dir, s.inv, s.oi, s.of);
     s.oct = (s.inv.x < 0.0f ? 1u : 0u) | (s.inv.y < 0.0f ? 2u : 0u) | (s.inv.z < 0.0f ? 4u : 0u);
     s.tmin = tmin;
     s.r = TraceResult{tmax, 0.f, 0.f, -1};
@@ -446,17 +461,18 @@ SST_D uint32_t visit8(const Trav8& s, uint32_t node) {
     return hm;
 }
 
-SST_D void trav8Begin(Trav8& s, const Bvh8 bvh, float3 org, float3 dir, float tmin, float tmax) {
+SST_D void trav8Begin(Trav8& s, const DevScene& sc, float3 org, float3 dir, float tmin, float tmax) {
+    const Bvh8 bvh = bvh8Of(sc);
     s.bvh = bvh;
     s.org = org;
     s.pre = rayPre(dir);
-    raySlabs(org, dir, s.inv, s.oi, s.of);
+    raySlabs(sc, org, dir, s.inv, s.oi, s.of);
     s.oct = (s.inv.x < 0.0f ? 1u : 0u) | (s.inv.y < 0.0f ? 2u : 0u) | (s.inv.z < 0.0f ? 4u : 0u);
     s.tmin = tmin;
     s.r = TraceResult{tmax, 0.f, 0.f, -1};
     s.sp = 0;
     s.node = 0;
-    s.done = bvh.nNodes8 == 0 || !(tmax > tmin) || originLost(org);
+    s.done = bvh.nNodes8 == 0 || !(tmax > tmin) || originLost(org) || noShear(s.pre);
     s.mask = s.done ? 0u : visit8(s, 0u);  // the root's hit children
     if (!s.done && s.mask == 0u) s.done = true;
 }
@@ -516,14 +532,14 @@ template <int W> struct WideTrav;
 template <> struct WideTrav<4> {
     using State = Trav4;
     static constexpr int kStack = kMaxStack4;
-    SST_D static void begin(State& s, const DevScene& sc, float3 o, float3 d, float tmin, float tmax) { trav4Begin(s, bvh4Of(sc), o, d, tmin, tmax); }
+    SST_D static void begin(State& s, const DevScene& sc, float3 o, float3 d, float tmin, float tmax) { trav4Begin(s, sc, o, d, tmin, tmax); }
     template <bool ANY, int BLOCK, int SSTACK>
     SST_D static bool run(State& s, int* sstack, int* lstack, int* err, int pause) { return trav4Run<ANY, BLOCK, SSTACK>(s, sstack, lstack, err, pause); }
 };
 template <> struct WideTrav<8> {
     using State = Trav8;
     static constexpr int kStack = kMaxStack;
-    SST_D static void begin(State& s, const DevScene& sc, float3 o, float3 d, float tmin, float tmax) { trav8Begin(s, bvh8Of(sc), o, d, tmin, tmax); }
+    SST_D static void begin(State& s, const DevScene& sc, float3 o, float3 d, float tmin, float tmax) { trav8Begin(s, sc, o, d, tmin, tmax); }
     template <bool ANY, int BLOCK, int SSTACK>
     SST_D static bool run(State& s, int* sstack, int* lstack, int* err, int pause) { return trav8Run<ANY, BLOCK, SSTACK>(s, sstack, lstack, err, pause); }
 };
@@ -605,7 +621,7 @@ __global__ void __launch_bounds__(BLOCK, (W == 8 ? SST_TRACE8_MIN_THREADS : SST_
             float4 o = ro[(size_t)i * rayStride], d = rd[(size_t)i * rayStride];
             uint32_t jb = rayJob ? rayJob[i] : 0u;
             const DevScene& sc = jobs[jb].sc;
-            TraceResult h = traverse<MODE != 0, BLOCK, SSTACK>(bvhOf(sc), f3(o), f3(d), o.w, d.w, sstack, &stats->errorFlags);
+            TraceResult h = traverse<MODE != 0, BLOCK, SSTACK>(sc, f3(o), f3(d), o.w, d.w, sstack, &stats->errorFlags);
             if (MODE == 0) {
                 hits[i] = make_float4(h.t, h.u, h.v, __int_as_float(h.tri));
             } else if (MODE == 1) {
