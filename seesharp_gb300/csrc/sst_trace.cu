@@ -95,17 +95,19 @@ SST_D Bvh bvhOf(const DevScene& sc) { return Bvh{sc.nodes, sc.triv, sc.nNodes}; 
 // of the tree while the rest of the GPU idled: on the 1M-triangle scene one path out of 67 million took
 // 300 to 800 ms of a render of 230 ms otherwise, a camera ray with one zero component 2.8 ms.
 // axisSlab gives that axis a finite inverse, a power of two, so that p * inv - o * inv is (p - o) * inv with
-// one rounding: its sign is exact.  The near plane is pulled in and the far plane pushed out by `push`: by
-// twice `reach`, which no distance to a box of the scene exceeds, so that they pass whenever the ray can
-// lie inside the slab; by what the component d moves the ray within that reach; and by two ulp of o * inv,
-// so that an origin exactly on a plane is inside (two triangles that share an edge in the ray's plane keep
-// it watertight).  Every box that holds a triangle the ray can meet passes, for directions of any length
-// (up to distances of 2.9e38, where push ends: with finite offsets an empty child's planes stay infinite).
-// Every other axis keeps the plain arithmetic, whatever the size of its component: a component is small
-// only against the others, as directions need not have unit length.
+// one rounding: its sign is exact.  The power keeps |o| * inv below 2^125: with a fixed one an origin beyond
+// 2^28 would push the near planes of every box out to infinity.  The near plane is pulled in and the far
+// plane pushed out by `push`: by twice `reach`, which no distance to a box of the scene exceeds, so that they
+// pass whenever the ray can lie inside the slab; by what the component d moves the ray within that reach;
+// and by two ulp of o * inv, so that an origin exactly on a plane is inside (two triangles that share an
+// edge in the ray's plane keep it watertight).  Every box that holds a triangle the ray can meet passes, for
+// directions of any length (up to distances of 2.9e38, where push ends: with finite offsets an empty
+// child's planes stay infinite).  Every other axis keeps the plain arithmetic, whatever the size of its
+// component: a component is small only against the others, as directions need not have unit length.
 SST_D void axisSlab(float o, float d, float reach, float& inv, float& oi, float& of) {
     if (fabsf(oi) < CUDART_INF_F) return;
-    inv = copysignf(1.2676506e30f, inv);  // 2^100
+    const int e = int(__float_as_uint(o) >> 23 & 255u) - 127;                    // |o| < 2^(e + 1)
+    inv = copysignf(__uint_as_float(uint32_t(min(100, 124 - e) + 127) << 23), inv);  // 2^100 for |o| < 2^25
     const float at = -o * inv;
     const float push = fminf(reach * (2.0f + fabsf(d * inv)) + fabsf(at) * 2.4e-7f, 2.9e38f);
     oi = at - push;

@@ -12,9 +12,12 @@ WIDTHS = (2, 4, 8)
 
 def _soup(centres, size, rng):
     n = len(centres)
-    V = (centres[:, None, :] + rng.uniform(-size, size, (n, 3, 3))).astype(np.float32)
+    return _scene((centres[:, None, :] + rng.uniform(-size, size, (n, 3, 3))).astype(np.float32))
+
+
+def _scene(V):
     sc = Scene()
-    m = Mesh(V.reshape(-1, 3), np.arange(3 * n, dtype=np.int32))
+    m = Mesh(V.reshape(-1, 3), np.arange(3 * len(V), dtype=np.int32))
     m.Material = DiffuseMaterial()
     sc.Meshes.append(m)
     sc.Emitters.append(DiffuseEmitter(Triangle(m, 0), RgbColor(1, 1, 1)))
@@ -112,3 +115,27 @@ def test_small_components_beside_ordinary_ones_hit_what_fp64_hits(width):
     assert np.array_equal(first_tri[ids[sure, 1]] + ids[sure, 0], tri[sure].astype(np.int64))
     assert (np.abs(hits[sure, 0] - t[sure]) <= 1e-5 * t[sure]).all()
     assert np.array_equal(occ != 0, ids[:, 0] >= 0)
+
+
+def test_hits_do_not_depend_on_the_scale_of_the_scene():
+    """A scene and ray origins scaled by a power of two (coordinates of up to 2e10) scale every distance
+    exactly.  A third of the rays run along an axis plane or an axis."""
+    n = 4000
+    want = None
+    for exponent in (0, 25, 30):
+        scale = np.float32(2.0 ** exponent)
+        rng = np.random.default_rng(6)
+        corners = rng.uniform(-20, 20, (4000, 1, 3)).astype(np.float32) + rng.uniform(-1, 1, (4000, 3, 3)).astype(np.float32)
+        sc = _scene(corners * scale)
+        org = rng.uniform(-20, 20, (n, 3)).astype(np.float32) * scale
+        d = rng.standard_normal((n, 3)).astype(np.float32)
+        k, first = np.arange(n), rng.integers(0, 3, n)
+        d[k[: n // 3], first[: n // 3]] = 0
+        d[k[: n // 6], (first[: n // 6] + 1) % 3] = -0.0
+        for width in WIDTHS:
+            hits, occ = _query(sc, _rays(org, d), width)
+            got = (hits[:, 0] / scale, hits[:, 1:3].view(np.uint32), _ids(hits), occ)
+            want = want or got
+            assert (_ids(hits)[: n // 6, 0] >= 0).any()
+            for a, b in zip(got, want):
+                assert np.array_equal(a, b), (exponent, width)
