@@ -527,10 +527,12 @@ void ensureBvh8(sst_scene* s) {
     int n8 = 0, depth8 = 0;
     int rc = buildBvh8(s->nodes.as<float4>(), s->nNodes, s->nodes8.as<float4>(), scratch8.p, &n8, &depth8, st);
     if (rc != 0) fail(SST_ERR_CUDA, "8-wide BVH build failed (" + std::to_string(rc) + "): " + cudaGetErrorString(cudaGetLastError()));
-    s->bvh8Built = true;
-    s->nNodes8 = n8 >= (1 << 24) ? 0 : n8;
-    s->bvh8Depth = depth8;
-    s->dev.nodes8 = s->nNodes8 > 0 ? s->nodes8.as<float4>() : nullptr;
-    s->dev.nNodes8 = s->nNodes8;
+    const int fits = n8 >= (1 << 24) ? 0 : n8;
+    s->dev.nodes8 = fits > 0 ? s->nodes8.as<float4>() : nullptr;
+    s->dev.nNodes8 = fits;
     uploadQueryJob(s);
+    // only now: a failure above leaves the scene traversed 4-wide, and the next call builds it again
+    s->nNodes8 = fits;
+    s->bvh8Depth = depth8;
+    s->bvh8Built = true;
 }

@@ -356,6 +356,7 @@ struct sst_scene {
     // device
     DevBuf nodes, nodes4, nodes8, triv, triN, triAux, triVtx, vnrm, vuv, mats, texs, texData, ems, envImg, envRowCdf, envColCdf, envHasCol, envRowMarg, queryJob;
     DevScene dev{};
+    DevJob queryJobHost{};  // what queryJob holds
     int nTri = 0, nNodes = 0, bvhDepth = 0, nNodes4 = 0, bvh4Depth = 0, nNodes8 = 0, bvh8Depth = 0;
     bool bvh8Built = false;  // the 8-wide BVH of the committed geometry exists (ensureBvh8)
     // adjoint: per-path radiance of the last sst_forward and its settings

@@ -3,12 +3,13 @@
 #include "sst_host.h"
 
 // The scene's one-entry job table (for the ray-query entry points), uploaded whenever its record
-// changes: at a commit and when the 8-wide BVH is built.
+// changes: at a commit and when the 8-wide BVH is built.  Its source stays in the scene, as the copy may
+// read it after this returns.
 void uploadQueryJob(sst_scene* s) {
-    DevJob j{};
-    j.sc = s->dev;
+    s->queryJobHost = DevJob{};
+    s->queryJobHost.sc = s->dev;
     s->queryJob.ensure(sizeof(DevJob));
-    CUDA_CHECK(cudaMemcpyAsync(s->queryJob.p, &j, sizeof(DevJob), cudaMemcpyHostToDevice, s->ctx->stream));
+    CUDA_CHECK(cudaMemcpyAsync(s->queryJob.p, &s->queryJobHost, sizeof(DevJob), cudaMemcpyHostToDevice, s->ctx->stream));
 }
 
 // Queries of up to this many rays between host arrays go through page-locked memory that the kernels

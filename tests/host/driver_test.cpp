@@ -1,0 +1,120 @@
+// Tests of the host driver (the C ABI without its kernels) over the CPU runtime of fake_cuda.h.  The kernel
+// launches are recorded or do nothing.  Usage: driver_test <name>; exit status 0 when it holds.
+#include <cstdio>
+#include <cstring>
+#include <map>
+#include <string>
+#include <vector>
+
+#include "../../seesharp_gb300/csrc/sst_host.h"
+#include "fake_cuda.h"
+
+#define EXPECT(c)                                                             \
+    do {                                                                      \
+        if (!(c)) {                                                           \
+            std::printf("%s:%d: %s does not hold\n", __FILE__, __LINE__, #c); \
+            return 1;                                                         \
+        }                                                                     \
+    } while (0)
+
+// ---- kernel launches --------------------------------------------------------------------------
+struct Query {
+    const float4* rays;
+    const int* occl;
+    DevScene scene;  // the job table's record, as the kernel finds it
+    std::vector<char> read;  // the rays, as the kernel finds them
+};
+static std::vector<Query> g_queries;
+
+namespace sst {
+size_t lbvhScratchBytes(int) { return 256; }
+size_t bvh4ScratchBytes(int) { return 256; }
+size_t bvh8ScratchBytes(int) { return 256; }
+int buildLbvh(const float4*, int, float4*, int*, void*, size_t, int* nodes, int* depth, cudaStream_t, int) { return *nodes = 1, *depth = 0, 0; }
+int buildBvh4(const float4*, int, float4*, void*, int* nodes, int* depth, cudaStream_t) { return *nodes = 1, *depth = 1, 0; }
+int buildBvh8(const float4*, int, float4*, void*, int* nodes, int* depth, cudaStream_t) { return *nodes = 1, *depth = 1, 0; }
+void launch_leaf_gather(const int*, int, const float4*, const float4*, const int4*, const int4*, float4*, float4*, int4*, int4*, cudaStream_t) {}
+void launch_env_build(const float4*, int, int, float*, float*, int*, float*, cudaStream_t) {}
+void launch_camera(const DevJob*, const WaveChunk*, const WaveDesc*, const int*, const PathBuf&, int*, int, cudaStream_t) {}
+void launch_light_start(const DevJob*, const LightParams&, const LightPathBuf&, int*, const LightVerts&, int*, cudaStream_t) {}
+void launch_light_walk(const DevJob*, const LightParams&, const LightPathBuf&, const LightPathBuf&, const float4*, const int*, int*, const LightVerts&, int*,
+                       int, cudaStream_t) {}
+void launch_error_trim(const float*, int, int, int, double*, cudaStream_t) {}
+void launch_variance_finish(const float*, const float*, int, int, float*, double*, cudaStream_t) {}
+void launch_film_fold(const DevJob*, const WaveChunk*, const WaveDesc*, int*, const float*, DevStats*, int, int, cudaStream_t) {}
+bool traceTuningValid(const TraceTuning&) { return true; }
+int traceGrid(const TraceTuning&) { return 152; }
+int traceMaxBlocksPerSM(const TraceTuning&) { return 1; }
+void launch_trace_closest(const TraceTuning&, const DevJob*, const uint32_t*, const float4*, const float4*, const int*, int*, float4*, DevStats*,
+                          cudaStream_t) {}
+void launch_trace_shadow(const TraceTuning&, const DevJob*, const uint32_t*, const float4*, const float4*, const int*, const int*, int*, float4*, DevStats*,
+                         cudaStream_t) {}
+void launch_trace_query(const TraceTuning&, const DevJob* jobs, const float4* rays, int n, int*, float4*, int* occl, DevStats*, bool any, cudaStream_t) {
+    fake::enqueue([=] {
+        Query q{rays, occl, jobs[0].sc, {}};
+        const char* r = reinterpret_cast<const char*>(rays);
+        q.read.assign(r, r + size_t(n) * sizeof(SstRay));
+        if (any) std::fill(occl, occl + n, 1);
+        g_queries.push_back(q);
+    });
+}
+void launch_wave_advance(int*, int, cudaStream_t) {}
+void launch_partition(bool, const uint32_t*, const float4*, const int*, int*, int*, int, cudaStream_t) {}
+bool shadeBlocksValid(int) { return true; }
+void launch_shade(int, bool, bool, int, const DevJob*, const PathBuf&, const PathBuf&, const float4*, float4*, float4*, int, float4*, float4*, int*,
+                  uint32_t*, const int*, int*, int*, float*, DevStats*, int, cudaStream_t) {}
+void launch_shade_pyramid(int, const DevJob*, const PathBuf&, const PathBuf&, const float4*, float4*, int, float4*, float4*, int*, uint32_t*, const int*,
+                          int*, int*, float*, DevStats*, const PyrArgs&, int, cudaStream_t) {}
+void launch_hit_expand(const DevScene&, const float4*, int, SstHitDev*, cudaStream_t) {}
+void launch_debug_material_eval(const DevScene&, int, int, const float*, const float*, const float*, float*, float*, cudaStream_t) {}
+void launch_debug_material_sample(const DevScene&, int, int, const float*, const float*, const float*, float*, float*, float*, cudaStream_t) {}
+void launch_debug_env(const DevScene&, int, const float*, float*, float*, float*, const float*, float*, float*, cudaStream_t) {}
+void launch_debug_rng(uint32_t, uint32_t, int, const uint32_t*, int, uint32_t*, cudaStream_t) {}
+void launch_debug_camera(const DevScene&, int, const float*, float*, float*, cudaStream_t) {}
+}  // namespace sst
+
+// ---- a scene of one emissive triangle ------------------------------------------------------------
+static sst_scene* makeScene(sst_ctx* ctx) {
+    sst_scene* s = nullptr;
+    if (sst_scene_create(ctx, &s) != SST_OK) return nullptr;
+    const float base[3] = {0.5f, 0.5f, 0.5f}, V[9] = {0, 0, 0, 1, 0, 0, 0, 1, 0}, rad[3] = {1, 1, 1};
+    const float w2c[16] = {1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, 0, 0, 0, -5, 1};
+    const int32_t I[3] = {0, 1, 2};
+    int32_t id = 0, first = 0, count = 0;
+    if (sst_scene_add_material_diffuse(s, base, -1, 0, &id) != SST_OK) return nullptr;
+    if (sst_scene_add_mesh(s, V, 3, I, 1, nullptr, nullptr, id, &id) != SST_OK) return nullptr;
+    if (sst_scene_add_emitters(s, id, nullptr, 0, rad, -1.0f, &first, &count) != SST_OK) return nullptr;
+    if (sst_scene_set_camera(s, w2c, 40.0f) != SST_OK) return nullptr;
+    return s;
+}
+
+// ---- the tests --------------------------------------------------------------------------------------
+// The job table that queries keep is read from memory that is still there, also when it is uploaded
+// again because a query has built the 8-wide BVH.
+static int queryJob(sst_ctx* ctx) {
+    SstTuning t;
+    EXPECT(sst_get_tuning(ctx, &t) == SST_OK);
+    sst_scene* s = makeScene(ctx);
+    EXPECT(s && sst_scene_commit(s, 8, 8) == SST_OK);
+    SstRay ray{};
+    ray.tmax = 1.0f;
+    int32_t occ = -1;
+    for (int width : {4, 8, 8}) {
+        t.traceBvhWidth = width;
+        EXPECT(sst_set_tuning(ctx, &t) == SST_OK);
+        EXPECT(sst_occluded(s, &ray, 1, &occ, SST_MEM_HOST) == SST_OK && occ == 1);
+        const DevScene& got = g_queries.back().scene;
+        EXPECT(got.triv == s->triv.as<float4>() && got.nodes4 == s->nodes4.as<float4>() && got.nNodes4 == 1 && got.nTri == 1);
+        EXPECT(got.nNodes8 == (width == 8 ? 1 : 0) && got.nodes8 == (width == 8 ? s->nodes8.as<float4>() : nullptr));
+    }
+    return sst_scene_destroy(s);
+}
+
+int main(int argc, char** argv) {
+    const std::map<std::string, int (*)(sst_ctx*)> tests = {{"query_job", queryJob}};
+    const auto it = argc > 1 ? tests.find(argv[1]) : tests.end();
+    sst_ctx* ctx = nullptr;
+    EXPECT(it != tests.end() && sst_create(0, &ctx) == SST_OK);
+    const int rc = it->second(ctx);
+    return rc ? rc : sst_destroy(ctx);
+}
