@@ -21,7 +21,7 @@ void uploadQueryJob(sst_scene* s) {
 constexpr int kTraceInPlace = 2048, kOcclInPlace = 8192;
 
 // Trace / IsOccluded over n rays.  The traversal reads the SstRay records where they are (device
-// arrays on a 16-byte boundary) or from one copy of them; sst_trace's SstHit records are expanded on the
+// arrays on a 16-byte boundary, apart from the results) or from one copy of them; sst_trace's SstHit records are expanded on the
 // device from the traversal's (t, u, v, triangle) records.  The buffers are the context's and only
 // grow, so repeated queries of the same size allocate nothing.
 static void runQuery(sst_scene* s, const SstRay* rays, int n, SstHit* hits, int32_t* occl, int memory, bool anyHit) {
@@ -52,7 +52,10 @@ static void runQuery(sst_scene* s, const SstRay* rays, int n, SstHit* hits, int3
         dRays = stage + 256;
         dOut = stage + 256 + rayBytes;
     } else {
-        if (!device || (reinterpret_cast<uintptr_t>(rays) & 15u)) {
+        // device rays that the results overlay are copied too: a ray's flag may be written before another ray is read
+        const char *r = reinterpret_cast<const char*>(rays), *o = static_cast<const char*>(userOut);
+        const bool overlaid = o < r + rayBytes && r < o + outBytes;
+        if (!device || overlaid || (reinterpret_cast<uintptr_t>(rays) & 15u)) {
             c->qRays.ensure(rayBytes);
             CUDA_CHECK(cudaMemcpyAsync(c->qRays.p, rays, rayBytes, device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
             dRays = c->qRays.p;

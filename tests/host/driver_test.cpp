@@ -110,8 +110,37 @@ static int queryJob(sst_ctx* ctx) {
     return sst_scene_destroy(s);
 }
 
+// Device results that overlay the rays are written only once the rays have been read.
+static int overlay(sst_ctx* ctx) {
+    sst_scene* s = makeScene(ctx);
+    EXPECT(s && sst_scene_commit(s, 8, 8) == SST_OK);
+    const int n = 100;
+    SstRay* rays = nullptr;
+    EXPECT(cudaMalloc(reinterpret_cast<void**>(&rays), n * sizeof(SstRay)) == cudaSuccess);
+    for (int k = 0; k < n; ++k) rays[k] = SstRay{{float(k), 0, 0}, 0, {0, 0, 1}, 1};
+    const std::vector<SstRay> before(rays, rays + n);
+    int32_t* const at[] = {reinterpret_cast<int32_t*>(rays), reinterpret_cast<int32_t*>(rays + n / 2), reinterpret_cast<int32_t*>(rays + n) - 1};
+    const int count[] = {n, 60, 1};
+    for (int k = 0; k < 3; ++k) {
+        std::copy(before.begin(), before.end(), rays);
+        EXPECT(sst_occluded(s, rays, count[k], at[k], SST_MEM_DEVICE) == SST_OK);
+        const Query& q = g_queries.back();
+        const char *r0 = reinterpret_cast<const char*>(q.rays), *r1 = r0 + count[k] * sizeof(SstRay);
+        const char *o0 = reinterpret_cast<const char*>(q.occl), *o1 = o0 + count[k] * sizeof(int32_t);
+        EXPECT(q.occl == at[k] && (o1 <= r0 || r1 <= o0));
+        EXPECT(std::memcmp(q.read.data(), before.data(), q.read.size()) == 0);
+    }
+    // apart: read where they are
+    int32_t* occ = nullptr;
+    EXPECT(cudaMalloc(reinterpret_cast<void**>(&occ), n * sizeof(int32_t)) == cudaSuccess);
+    EXPECT(sst_occluded(s, rays, n, occ, SST_MEM_DEVICE) == SST_OK && g_queries.back().rays == reinterpret_cast<const float4*>(rays));
+    cudaFree(occ);
+    cudaFree(rays);
+    return sst_scene_destroy(s);
+}
+
 int main(int argc, char** argv) {
-    const std::map<std::string, int (*)(sst_ctx*)> tests = {{"query_job", queryJob}};
+    const std::map<std::string, int (*)(sst_ctx*)> tests = {{"query_job", queryJob}, {"overlay", overlay}};
     const auto it = argc > 1 ? tests.find(argv[1]) : tests.end();
     sst_ctx* ctx = nullptr;
     EXPECT(it != tests.end() && sst_create(0, &ctx) == SST_OK);

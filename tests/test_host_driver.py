@@ -43,3 +43,7 @@ def run(driver, name, **env):
 
 def test_query_job_table_is_uploaded_from_memory_that_stays(driver):
     run(driver, "query_job")
+
+
+def test_results_may_overlay_the_rays(driver):
+    run(driver, "overlay")
