@@ -163,18 +163,22 @@ void parallelRanges(size_t n, size_t minPerThread, F fn) {
 // byte written back, which costs two faults per page: the read maps the zero page, and replacing it
 // invalidates the GPU's translations too (61 MB of light paths: 12 ms with one thread, 25 ms with eight,
 // against 1.3 ms populated).  renderJobs starts it once the first wave is on its way: before the
-// launches a thread's start (about 50 us) is time in which the GPU has nothing to do.
+// launches a thread's start (about 50 us) is time in which the GPU has nothing to do.  Work is in flight
+// then, so start() does not throw: where no thread can be started, the read-back faults the pages in.
 class HostPrefault {
 public:
     void add(void* p, size_t bytes) {
         if (p && bytes) bufs_.push_back({static_cast<char*>(p), bytes});
     }
-    void start() {
+    void start() noexcept {
         size_t total = 0;
         for (auto& b : bufs_) total += b.second;
         if (total == 0) return;
         const size_t n = std::min<size_t>(kThreads, (total + kPerThread - 1) / kPerThread), share = (total + n - 1) / n;
-        for (size_t t = 0; t < n; ++t) th_.emplace_back([this, b = t * share, e = std::min(total, (t + 1) * share)] { run(b, e); });
+        try {
+            for (size_t t = 0; t < n; ++t) th_.emplace_back([this, b = t * share, e = std::min(total, (t + 1) * share)] { run(b, e); });
+        } catch (const std::exception&) {
+        }
     }
     void finish() {
         for (auto& t : th_) t.join();

@@ -139,8 +139,32 @@ static int overlay(sst_ctx* ctx) {
     return sst_scene_destroy(s);
 }
 
+static SstPathTracerParams params(int spp) {
+    SstPathTracerParams p{};
+    p.width = p.height = 8;
+    p.totalSpp = spp;
+    p.maxDepth = 3;
+    p.numShadowRays = 1;
+    return p;
+}
+
+// Output pages are populated by helper threads; a process that can start no more threads renders all the same.
+static int threads(sst_ctx* ctx) {
+    sst_scene* s = makeScene(ctx);
+    EXPECT(s && sst_scene_commit(s, 8, 8) == SST_OK);
+    const SstPathTracerParams p = params(2);
+    std::vector<float> film(3 * 64);
+    std::vector<SstPathVertex> v(10 * 4);
+    std::vector<int32_t> len(10);
+    fake::threadsFail = true;
+    EXPECT(sst_render(s, &p, film.data(), SST_MEM_HOST, nullptr) == SST_OK);
+    EXPECT(sst_trace_light_paths(s, 1, 0, 10, 3, v.data(), len.data(), SST_MEM_HOST, nullptr) == SST_OK);
+    fake::threadsFail = false;
+    return sst_scene_destroy(s);
+}
+
 int main(int argc, char** argv) {
-    const std::map<std::string, int (*)(sst_ctx*)> tests = {{"query_job", queryJob}, {"overlay", overlay}};
+    const std::map<std::string, int (*)(sst_ctx*)> tests = {{"query_job", queryJob}, {"overlay", overlay}, {"threads", threads}};
     const auto it = argc > 1 ? tests.find(argv[1]) : tests.end();
     sst_ctx* ctx = nullptr;
     EXPECT(it != tests.end() && sst_create(0, &ctx) == SST_OK);

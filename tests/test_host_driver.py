@@ -47,3 +47,7 @@ def test_query_job_table_is_uploaded_from_memory_that_stays(driver):
 
 def test_results_may_overlay_the_rays(driver):
     run(driver, "overlay")
+
+
+def test_renders_without_helper_threads(driver):
+    run(driver, "threads")
