@@ -277,6 +277,20 @@ void renderJobs(sst_ctx* c, std::vector<JobIn>& jobs, SstRenderStats* out, bool 
             if (tab[j].lay.aovAlbedo) tab[j].lay.aovSamples = sk.aov.as<float>();
         setJobs[k] = reinterpret_cast<const DevJob*>(c->renderBlock.as<char>() + oJobs[k]);
     }
+    // A render that fails from here on waits for what it has launched: it reads the scenes, whose memory is
+    // given back in the order of the context's stream alone, and the tables.
+    struct Drain {
+        sst_ctx* c;
+        int before = std::uncaught_exceptions();
+        ~Drain() {
+            if (std::uncaught_exceptions() == before) return;
+            for (WaveStore& s : c->store) {
+                cudaStreamSynchronize(s.run);
+                cudaStreamSynchronize(s.side);
+            }
+            cudaStreamSynchronize(c->stream);
+        }
+    } drain{c};
     CUDA_CHECK(cudaMemcpyAsync(c->renderBlock.p, hostBlock, blockBytes, cudaMemcpyHostToDevice, st));
     if (!staged) CUDA_CHECK(cudaStreamSynchronize(st));
     const WaveChunk* dch = reinterpret_cast<const WaveChunk*>(c->renderBlock.as<char>() + oChunks);

@@ -163,8 +163,25 @@ static int threads(sst_ctx* ctx) {
     return sst_scene_destroy(s);
 }
 
+// A render that fails midway has waited for what it launched: nothing runs on after it returns.
+static int failedRender(sst_ctx* ctx) {
+    sst_scene* s = makeScene(ctx);
+    EXPECT(s && sst_scene_commit(s, 8, 8) == SST_OK);
+    const SstPathTracerParams p = params(2);
+    std::vector<float> film(3 * 64);
+    bool failed = true;
+    for (int k = 1; failed; ++k) {
+        fake::failingRecord = k;
+        failed = sst_render(s, &p, film.data(), SST_MEM_HOST, nullptr) != SST_OK;
+        EXPECT(fake::pending() == 0);
+        EXPECT(k > 2 || failed);
+    }
+    fake::failingRecord = 0;
+    return sst_scene_destroy(s);
+}
+
 int main(int argc, char** argv) {
-    const std::map<std::string, int (*)(sst_ctx*)> tests = {{"query_job", queryJob}, {"overlay", overlay}, {"threads", threads}};
+    const std::map<std::string, int (*)(sst_ctx*)> tests = {{"query_job", queryJob}, {"overlay", overlay}, {"threads", threads}, {"failed_render", failedRender}};
     const auto it = argc > 1 ? tests.find(argv[1]) : tests.end();
     sst_ctx* ctx = nullptr;
     EXPECT(it != tests.end() && sst_create(0, &ctx) == SST_OK);

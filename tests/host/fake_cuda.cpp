@@ -16,6 +16,7 @@ struct CUmemPoolHandle_st {
 namespace fake {
 size_t budget = size_t(1) << 40;
 bool threadsFail = false;
+int failingRecord = 0;
 namespace {
 std::vector<std::function<void()>> queue;
 struct Block {
@@ -77,6 +78,7 @@ template <class T> cudaError_t dropped(T h) {
     return cudaSuccess;
 }
 }  // namespace
+size_t pending() { return queue.size(); }
 void enqueue(std::function<void()> op) { queue.push_back(std::move(op)); }
 size_t used() {
     size_t n = 0;
@@ -112,7 +114,7 @@ cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cu
 cudaError_t cudaEventCreate(cudaEvent_t* e) { return handle(e); }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return handle(e); }
 cudaError_t cudaEventDestroy(cudaEvent_t e) { return dropped(e); }
-cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return failingRecord > 0 && --failingRecord == 0 ? set(cudaErrorUnknown) : cudaSuccess; }
 cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { return *ms = 1.0f, cudaSuccess; }
 cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return set(cudaErrorNotSupported); }
 cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t*) { return set(cudaErrorNotSupported); }

@@ -13,4 +13,6 @@ void enqueue(std::function<void()> op);
 extern size_t budget;       // bytes of device memory
 size_t used();              // live blocks and what pools hold
 extern bool threadsFail;    // pthread_create returns EAGAIN
+size_t pending();           // operations that no wait has run yet
+extern int failingRecord;   // the event record, counted from now, that fails; 0: none
 }  // namespace fake

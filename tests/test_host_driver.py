@@ -51,3 +51,7 @@ def test_results_may_overlay_the_rays(driver):
 
 def test_renders_without_helper_threads(driver):
     run(driver, "threads")
+
+
+def test_a_failed_render_has_waited_for_its_launches(driver):
+    run(driver, "failed_render")
