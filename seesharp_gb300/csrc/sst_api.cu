@@ -9,6 +9,15 @@
 
 thread_local std::string g_lastError;
 
+// The scene pools of all contexts, so that an allocation that fails in one of them, or in a context's own
+// buffers, can have what they hold unused.
+static std::mutex g_poolLock;
+static std::vector<cudaMemPool_t> g_pools;
+void trimScenePools() {
+    std::lock_guard<std::mutex> g(g_poolLock);
+    for (cudaMemPool_t p : g_pools) cudaMemPoolTrimTo(p, 0);
+}
+
 // ---------------------------------------------------------------------------------------------
 // C ABI
 // ---------------------------------------------------------------------------------------------
@@ -57,6 +66,8 @@ int sst_create(int32_t device, sst_ctx** out) {
             CUDA_CHECK(cudaMemPoolCreate(&c->scenePool, &props));
             uint64_t keep = kScenePoolBytes;
             CUDA_CHECK(cudaMemPoolSetAttribute(c->scenePool, cudaMemPoolAttrReleaseThreshold, &keep));
+            std::lock_guard<std::mutex> g(g_poolLock);
+            g_pools.push_back(c->scenePool);
         }
         *out = c.release();
     });
@@ -81,7 +92,13 @@ int sst_destroy(sst_ctx* ctx) {
             if (ws.side) cudaStreamDestroy(ws.side);
             if (ws.run) cudaStreamDestroy(ws.run);
         }
-        if (ctx->scenePool) cudaMemPoolDestroy(ctx->scenePool);
+        if (ctx->scenePool) {
+            {
+                std::lock_guard<std::mutex> g(g_poolLock);
+                g_pools.erase(std::remove(g_pools.begin(), g_pools.end(), ctx->scenePool), g_pools.end());
+            }
+            cudaMemPoolDestroy(ctx->scenePool);
+        }
         cudaStreamDestroy(ctx->stream);
         delete ctx;
     });

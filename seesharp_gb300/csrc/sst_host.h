@@ -70,8 +70,12 @@ template <class F> int guarded(F&& f) {
 // ---------------------------------------------------------------------------------------------
 // device buffers
 // ---------------------------------------------------------------------------------------------
+// Gives the unused memory of all contexts' scene pools back to their devices (sst_api.cu).
+void trimScenePools();
+
 // A buffer given a pool takes blocks of up to kPooledBytes from it, ordered on the pool's stream; larger
-// ones, and buffers without a pool, are allocated on their own.
+// ones, and buffers without a pool, are allocated on their own.  Where the device is out of memory, what
+// the pools hold unused is given back first.
 constexpr size_t kPooledBytes = size_t(256) << 20;
 struct DevBuf {
     void* p = nullptr;
@@ -97,10 +101,18 @@ struct DevBuf {
         if (b <= bytes) return;
         release();
         pooled = pool && b <= kPooledBytes;
-        if (pooled) CUDA_CHECK(cudaMallocFromPoolAsync(&p, b, pool, poolStream));
-        else CUDA_CHECK(cudaMalloc(&p, b));
+        cudaError_t e = allocate(b);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            if (pool) cudaStreamSynchronize(poolStream);  // what was freed in its order is free now
+            trimScenePools();
+            e = allocate(b);
+            if (e != cudaSuccess) cudaGetLastError();  // reported below, not by the next launch
+        }
+        CUDA_CHECK(e);
         bytes = b;
     }
+    cudaError_t allocate(size_t b) { return pooled ? cudaMallocFromPoolAsync(&p, b, pool, poolStream) : cudaMalloc(&p, b); }
     template <class T> void upload(const std::vector<T>& v, cudaStream_t s) {
         ensure(std::max<size_t>(1, v.size() * sizeof(T)));
         if (!v.empty()) CUDA_CHECK(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s));

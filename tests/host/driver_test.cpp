@@ -180,8 +180,39 @@ static int failedRender(sst_ctx* ctx) {
     return sst_scene_destroy(s);
 }
 
+// Memory that a pool holds unused does not make another allocation fail, in or outside the pool, nor
+// leave an error behind.
+static int outOfMemory(sst_ctx* ctx) {
+    const size_t MB = size_t(1) << 20;
+    const size_t own = fake::used();
+    fake::budget = own + 512 * MB;
+    {
+        DevBuf a, b, c, d;
+        for (DevBuf* x : {&a, &b, &c}) x->use(ctx->scenePool, ctx->stream);
+        a.ensure(200 * MB);
+        b.ensure(200 * MB);
+        EXPECT(cudaStreamSynchronize(ctx->stream) == cudaSuccess);
+        a.release();
+        d.ensure(300 * MB);  // the context's own: 200 MB are in use and 200 MB held
+        EXPECT(d.p && cudaGetLastError() == cudaSuccess);
+        d.release();
+        a.ensure(200 * MB);
+        a.release();
+        c.ensure(256 * MB);
+        EXPECT(c.p && cudaGetLastError() == cudaSuccess);
+        bool refused = false;
+        try {
+            d.ensure(300 * MB);
+        } catch (const SstException& e) {
+            refused = e.code == SST_ERR_OUT_OF_MEMORY;
+        }
+        EXPECT(refused && !d.p && d.bytes == 0 && cudaGetLastError() == cudaSuccess);
+    }
+    return 0;
+}
+
 int main(int argc, char** argv) {
-    const std::map<std::string, int (*)(sst_ctx*)> tests = {{"query_job", queryJob}, {"overlay", overlay}, {"threads", threads}, {"failed_render", failedRender}};
+    const std::map<std::string, int (*)(sst_ctx*)> tests = {{"query_job", queryJob}, {"overlay", overlay}, {"threads", threads}, {"failed_render", failedRender}, {"out_of_memory", outOfMemory}};
     const auto it = argc > 1 ? tests.find(argv[1]) : tests.end();
     sst_ctx* ctx = nullptr;
     EXPECT(it != tests.end() && sst_create(0, &ctx) == SST_OK);

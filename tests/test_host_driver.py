@@ -55,3 +55,7 @@ def test_renders_without_helper_threads(driver):
 
 def test_a_failed_render_has_waited_for_its_launches(driver):
     run(driver, "failed_render")
+
+
+def test_unused_pool_memory_does_not_fail_allocations(driver):
+    run(driver, "out_of_memory")
