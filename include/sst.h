@@ -118,7 +118,12 @@ int sst_version(int32_t* major, int32_t* minor);
 /* Copies the calling thread's last error message (NUL-terminated, truncated to size). */
 int sst_last_error(char* buffer, size_t size);
 
-/* Creates a context on a CUDA device: one stream, the device kernels, scratch pools. */
+/* Creates a context on a CUDA device: one stream, the device kernels, scratch pools.
+ * A context keeps device memory until it is destroyed: the wave, query and layer buffers at the largest
+ * size that its calls needed, and up to 256 MB of the memory of destroyed scenes for the next ones.  The
+ * environment variable SST_SCENE_POOL_MB, read here, sets the latter in megabytes; with 0 a destroyed
+ * scene's memory goes back to the device at once.  An allocation of this library that fails gives it back
+ * and is tried again. */
 int sst_create(int32_t device, sst_ctx** out);
 int sst_destroy(sst_ctx* ctx);
 

@@ -58,13 +58,14 @@ int sst_create(int32_t device, sst_ctx** out) {
         CUDA_CHECK(cudaMallocHost(&c->pinnedCount, sizeof(int) * 4));
         int pools = 0;
         CUDA_CHECK(cudaDeviceGetAttribute(&pools, cudaDevAttrMemoryPoolsSupported, device));
-        if (pools) {
+        const char* poolEnv = getenv("SST_SCENE_POOL_MB");
+        uint64_t keep = poolEnv ? uint64_t(std::max(0ll, atoll(poolEnv))) << 20 : kScenePoolBytes;
+        if (pools && keep > 0) {
             cudaMemPoolProps props{};
             props.allocType = cudaMemAllocationTypePinned;
             props.location.type = cudaMemLocationTypeDevice;
             props.location.id = device;
             CUDA_CHECK(cudaMemPoolCreate(&c->scenePool, &props));
-            uint64_t keep = kScenePoolBytes;
             CUDA_CHECK(cudaMemPoolSetAttribute(c->scenePool, cudaMemPoolAttrReleaseThreshold, &keep));
             std::lock_guard<std::mutex> g(g_poolLock);
             g_pools.push_back(c->scenePool);
@@ -115,8 +116,10 @@ int sst_scene_destroy(sst_scene* scene) {
     return guarded([&] {
         if (!scene) return;
         cudaSetDevice(scene->ctx->device);
-        cudaStreamSynchronize(scene->ctx->stream);
+        const cudaStream_t st = scene->ctx->stream;
+        cudaStreamSynchronize(st);
         delete scene;
+        cudaStreamSynchronize(st);  // the wait returns what the pool holds beyond its bound
     });
 }
 

@@ -77,6 +77,11 @@ void trimScenePools();
 // ones, and buffers without a pool, are allocated on their own.  Where the device is out of memory, what
 // the pools hold unused is given back first.
 constexpr size_t kPooledBytes = size_t(256) << 20;
+// What a context's pool keeps unused unless SST_SCENE_POOL_MB says otherwise (0: no pool).  Scene.Prepare
+// of 10K / 102K / 614K / 1M / 2M triangles: 2.16 / 4.01 / 10.0 / 15.1 / 27.3 ms without a pool, 1.77 / 3.44 /
+// 8.85 / 13.9 / 26.9 ms with 128 MB, 1.75 / 3.39 / 8.71 / 13.7 / 26.6 with 256 MB, 1.76 / 3.41 / 8.66 / 13.5 /
+// 25.8 with 1 GB.
+constexpr uint64_t kScenePoolBytes = uint64_t(256) << 20;
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
@@ -260,8 +265,9 @@ struct sst_ctx {
     PinnedBuf commitStage;
     DevBuf commitTri[4], commitOrder, commitScratch, commitScratch4, commitScratch8;
     // The device memory of scenes that were destroyed, for the next ones: a program that prepares its
-    // scene anew for every frame would otherwise pay 17 allocations and 17 device-wide frees each time
-    // (1.8 ms of a 13.7 ms frame of 614K triangles).  It keeps at most kScenePoolBytes, and goes with the context.
+    // scene anew for every frame would otherwise pay 17 allocations and 17 device-wide frees each time.  It
+    // keeps at most kScenePoolBytes (the rest goes back when a scene is destroyed), gives that back too when
+    // an allocation fails, and goes with the context.
     cudaMemPool_t scenePool = nullptr;
     // wavefront buffers (store[1..] only while several waves are in flight)
     WaveStore store[kMaxWaveSets];
@@ -349,8 +355,6 @@ struct HostTexture {
     int w, h, ch, border;
     std::vector<float> data;
 };
-
-constexpr uint64_t kScenePoolBytes = uint64_t(1) << 30;
 
 struct sst_scene {
     explicit sst_scene(sst_ctx* c) : ctx(c) {

@@ -211,8 +211,24 @@ static int outOfMemory(sst_ctx* ctx) {
     return 0;
 }
 
+// A destroyed scene leaves at most the pool's bound behind, without another call.
+static int scenePool(sst_ctx* ctx) {
+    const size_t MB = size_t(1) << 20, own = fake::used();
+    const char* env = getenv("SST_SCENE_POOL_MB");
+    const size_t bound = env ? size_t(atoi(env)) * MB : 256 * MB;
+    sst_scene* s = makeScene(ctx);
+    EXPECT(s && sst_scene_commit(s, 8, 8) == SST_OK);
+    const size_t context = fake::used();  // the commit's scratch stays with the context
+    for (DevBuf* b : {&s->record, &s->gTex, &s->dLdI}) b->ensure(200 * MB);
+    EXPECT(fake::used() >= own + 600 * MB);
+    EXPECT(sst_scene_destroy(s) == SST_OK);
+    EXPECT(fake::pending() == 0 && fake::used() <= context + bound);
+    EXPECT(bound == 0 || fake::used() >= own + bound);
+    return 0;
+}
+
 int main(int argc, char** argv) {
-    const std::map<std::string, int (*)(sst_ctx*)> tests = {{"query_job", queryJob}, {"overlay", overlay}, {"threads", threads}, {"failed_render", failedRender}, {"out_of_memory", outOfMemory}};
+    const std::map<std::string, int (*)(sst_ctx*)> tests = {{"query_job", queryJob}, {"overlay", overlay}, {"threads", threads}, {"failed_render", failedRender}, {"out_of_memory", outOfMemory}, {"scene_pool", scenePool}};
     const auto it = argc > 1 ? tests.find(argv[1]) : tests.end();
     sst_ctx* ctx = nullptr;
     EXPECT(it != tests.end() && sst_create(0, &ctx) == SST_OK);

@@ -59,3 +59,8 @@ def test_a_failed_render_has_waited_for_its_launches(driver):
 
 def test_unused_pool_memory_does_not_fail_allocations(driver):
     run(driver, "out_of_memory")
+
+
+@pytest.mark.parametrize("megabytes", ["", "0", "100"])
+def test_destroyed_scenes_leave_at_most_the_bound(driver, megabytes):
+    run(driver, "scene_pool", **({"SST_SCENE_POOL_MB": megabytes} if megabytes else {}))
