@@ -21,6 +21,7 @@ int sst_forward_batch(sst_ctx* ctx, const SstRenderJob* jobs, int32_t numJobs, S
         CUDA_CHECK(cudaSetDevice(ctx->device));
         ctx->batchSig.clear();
         std::vector<JobIn> in;
+        const BatchFilms films{ctx};
         batchJobs(ctx, jobs, numJobs, in, true);
         if ((int)ctx->batchRecord.size() < numJobs) ctx->batchRecord.resize(numJobs);
         for (int j = 0; j < numJobs; ++j) {
@@ -58,6 +59,7 @@ int sst_backward_batch(sst_ctx* ctx, const SstRenderJob* jobs, int32_t numJobs, 
         CUDA_CHECK(cudaSetDevice(ctx->device));
         cudaStream_t st = ctx->stream;
         std::vector<JobIn> in;
+        const BatchFilms films{ctx};
         batchJobs(ctx, jobs, numJobs, in, true);
         if ((int)ctx->batchDLdI.size() < numJobs) ctx->batchDLdI.resize(numJobs);
         // gradient buffers of each distinct scene, zeroed once

@@ -421,6 +421,16 @@ template <class T> void hostCopy(T* h, const DevBuf& b, size_t n, cudaStream_t s
 }
 
 
+// Held by a batch call: the films staged for it stay with the context up to kBatchFilmBytes (5.6 million
+// pixels, whose paths take 20 ms and more); a larger buffer is given back when the call ends.
+constexpr size_t kBatchFilmBytes = size_t(64) << 20;
+struct BatchFilms {
+    sst_ctx* c;
+    ~BatchFilms() {
+        if (c->batchFilm.bytes > kBatchFilmBytes) c->batchFilm.release();
+    }
+};
+
 // ---- shared functions ------------------------------------------------------------------------
 // sst_commit.cu
 bool invert4(const float* m, float* out);  // 4x4 inverse (row-major); false when singular

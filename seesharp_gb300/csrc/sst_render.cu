@@ -1084,6 +1084,7 @@ int sst_render_batch(sst_ctx* ctx, const SstRenderJob* jobs, int32_t numJobs, Ss
         SstRenderStats total = emptyStats();
         std::vector<JobIn> in;
         auto t0 = std::chrono::steady_clock::now();
+        const BatchFilms films{ctx};
         batchJobs(ctx, jobs, numJobs, in, false);
         CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
         double fbMs = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();

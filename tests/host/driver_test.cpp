@@ -227,8 +227,34 @@ static int scenePool(sst_ctx* ctx) {
     return 0;
 }
 
+// The films that a batch stages on the device go back with the call when they are large.
+static int batchFilms(sst_ctx* ctx) {
+    const int W = 4096, H = 2048;
+    sst_scene *small = makeScene(ctx), *large = makeScene(ctx);
+    EXPECT(small && large && sst_scene_commit(small, 8, 8) == SST_OK && sst_scene_commit(large, W, H) == SST_OK);
+    std::vector<float> film(3 * size_t(W) * H), few(3 * 64);
+    SstRenderJob jobs[2] = {};
+    jobs[0].scene = large;
+    jobs[0].params = params(1);
+    jobs[0].params.width = W;
+    jobs[0].params.height = H;
+    jobs[0].film = film.data();
+    jobs[1].scene = small;
+    jobs[1].params = params(1);
+    jobs[1].film = few.data();
+    EXPECT(sst_render_batch(ctx, jobs + 1, 1, nullptr) == SST_OK);
+    EXPECT(ctx->batchFilm.bytes > 0 && ctx->batchFilm.bytes < 4096);
+    const void* kept = ctx->batchFilm.p;
+    EXPECT(sst_render_batch(ctx, jobs + 1, 1, nullptr) == SST_OK && ctx->batchFilm.p == kept);
+    EXPECT(sst_render_batch(ctx, jobs, 2, nullptr) == SST_OK);
+    EXPECT(ctx->batchFilm.bytes <= (size_t(64) << 20));
+    EXPECT(sst_forward_batch(ctx, jobs, 2, nullptr) == SST_OK);
+    EXPECT(ctx->batchFilm.bytes <= (size_t(64) << 20));
+    return sst_scene_destroy(small) + sst_scene_destroy(large);
+}
+
 int main(int argc, char** argv) {
-    const std::map<std::string, int (*)(sst_ctx*)> tests = {{"query_job", queryJob}, {"overlay", overlay}, {"threads", threads}, {"failed_render", failedRender}, {"out_of_memory", outOfMemory}, {"scene_pool", scenePool}};
+    const std::map<std::string, int (*)(sst_ctx*)> tests = {{"query_job", queryJob}, {"overlay", overlay}, {"threads", threads}, {"failed_render", failedRender}, {"out_of_memory", outOfMemory}, {"scene_pool", scenePool}, {"batch_films", batchFilms}};
     const auto it = argc > 1 ? tests.find(argv[1]) : tests.end();
     sst_ctx* ctx = nullptr;
     EXPECT(it != tests.end() && sst_create(0, &ctx) == SST_OK);

@@ -64,3 +64,7 @@ def test_unused_pool_memory_does_not_fail_allocations(driver):
 @pytest.mark.parametrize("megabytes", ["", "0", "100"])
 def test_destroyed_scenes_leave_at_most_the_bound(driver, megabytes):
     run(driver, "scene_pool", **({"SST_SCENE_POOL_MB": megabytes} if megabytes else {}))
+
+
+def test_large_batch_films_are_given_back(driver):
+    run(driver, "batch_films")
