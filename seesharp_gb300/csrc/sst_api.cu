@@ -59,16 +59,18 @@ int sst_create(int32_t device, sst_ctx** out) {
         int pools = 0;
         CUDA_CHECK(cudaDeviceGetAttribute(&pools, cudaDevAttrMemoryPoolsSupported, device));
         const char* poolEnv = getenv("SST_SCENE_POOL_MB");
-        uint64_t keep = poolEnv ? uint64_t(std::max(0ll, atoll(poolEnv))) << 20 : kScenePoolBytes;
-        if (pools && keep > 0) {
+        c->scenePool.stream = c->stream;
+        c->scenePool.keep = poolEnv ? size_t(std::max(0ll, atoll(poolEnv))) << 20 : kScenePoolBytes;
+        if (pools && c->scenePool.keep > 0) {
             cudaMemPoolProps props{};
             props.allocType = cudaMemAllocationTypePinned;
             props.location.type = cudaMemLocationTypeDevice;
             props.location.id = device;
-            CUDA_CHECK(cudaMemPoolCreate(&c->scenePool, &props));
-            CUDA_CHECK(cudaMemPoolSetAttribute(c->scenePool, cudaMemPoolAttrReleaseThreshold, &keep));
+            CUDA_CHECK(cudaMemPoolCreate(&c->scenePool.pool, &props));
+            uint64_t never = ~uint64_t(0);  // ScenePool::trim gives memory back
+            CUDA_CHECK(cudaMemPoolSetAttribute(c->scenePool.pool, cudaMemPoolAttrReleaseThreshold, &never));
             std::lock_guard<std::mutex> g(g_poolLock);
-            g_pools.push_back(c->scenePool);
+            g_pools.push_back(c->scenePool.pool);
         }
         *out = c.release();
     });
@@ -93,12 +95,12 @@ int sst_destroy(sst_ctx* ctx) {
             if (ws.side) cudaStreamDestroy(ws.side);
             if (ws.run) cudaStreamDestroy(ws.run);
         }
-        if (ctx->scenePool) {
+        if (ctx->scenePool.pool) {
             {
                 std::lock_guard<std::mutex> g(g_poolLock);
-                g_pools.erase(std::remove(g_pools.begin(), g_pools.end(), ctx->scenePool), g_pools.end());
+                g_pools.erase(std::remove(g_pools.begin(), g_pools.end(), ctx->scenePool.pool), g_pools.end());
             }
-            cudaMemPoolDestroy(ctx->scenePool);
+            cudaMemPoolDestroy(ctx->scenePool.pool);
         }
         cudaStreamDestroy(ctx->stream);
         delete ctx;
@@ -116,10 +118,10 @@ int sst_scene_destroy(sst_scene* scene) {
     return guarded([&] {
         if (!scene) return;
         cudaSetDevice(scene->ctx->device);
-        const cudaStream_t st = scene->ctx->stream;
-        cudaStreamSynchronize(st);
+        sst_ctx* const c = scene->ctx;
+        cudaStreamSynchronize(c->stream);
         delete scene;
-        cudaStreamSynchronize(st);  // the wait returns what the pool holds beyond its bound
+        c->scenePool.trim();
     });
 }
 
@@ -311,6 +313,7 @@ int sst_scene_commit(sst_scene* s, int32_t w, int32_t h) {
     return guarded([&] {
         if (!s) fail(SST_ERR_INVALID_ARGUMENT, "NULL scene");
         commitScene(s, w, h);
+        s->ctx->scenePool.trim();  // buffers that it grew
     });
 }
 

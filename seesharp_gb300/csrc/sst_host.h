@@ -82,42 +82,55 @@ constexpr size_t kPooledBytes = size_t(256) << 20;
 // 8.85 / 13.9 / 26.9 ms with 128 MB, 1.75 / 3.39 / 8.71 / 13.7 / 26.6 with 256 MB, 1.76 / 3.41 / 8.66 / 13.5 /
 // 25.8 with 1 GB.
 constexpr uint64_t kScenePoolBytes = uint64_t(256) << 20;
+struct ScenePool {
+    cudaMemPool_t pool = nullptr;
+    cudaStream_t stream = nullptr;
+    size_t live = 0;  // bytes of the buffers that hold memory of the pool
+    size_t keep = 0;
+    // Gives back what the pool holds beyond `keep` unused bytes.  (The pool's own release threshold counts
+    // the live buffers too: a program with several scenes would keep nothing of a destroyed one.)
+    void trim() {
+        if (!pool) return;
+        cudaStreamSynchronize(stream);  // what was freed in its order is free now
+        cudaMemPoolTrimTo(pool, live + keep);
+    }
+};
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
-    cudaMemPool_t pool = nullptr;
-    cudaStream_t poolStream = nullptr;
+    ScenePool* pool = nullptr;
     bool pooled = false;
     DevBuf() = default;
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
     ~DevBuf() { release(); }
-    void use(cudaMemPool_t mp, cudaStream_t s) {
-        pool = mp;
-        poolStream = s;
-    }
     void release() {
-        if (p && pooled) cudaFreeAsync(p, poolStream);
-        else if (p) cudaFree(p);
+        if (p && pooled) {
+            cudaFreeAsync(p, pool->stream);
+            pool->live -= bytes;
+        } else if (p) {
+            cudaFree(p);
+        }
         p = nullptr;
         bytes = 0;
     }
     void ensure(size_t b) {
         if (b <= bytes) return;
         release();
-        pooled = pool && b <= kPooledBytes;
+        pooled = pool && pool->pool && b <= kPooledBytes;
         cudaError_t e = allocate(b);
         if (e == cudaErrorMemoryAllocation) {
             cudaGetLastError();
-            if (pool) cudaStreamSynchronize(poolStream);  // what was freed in its order is free now
+            if (pool) cudaStreamSynchronize(pool->stream);  // what was freed in its order is free now
             trimScenePools();
             e = allocate(b);
             if (e != cudaSuccess) cudaGetLastError();  // reported below, not by the next launch
         }
         CUDA_CHECK(e);
         bytes = b;
+        if (pooled) pool->live += b;
     }
-    cudaError_t allocate(size_t b) { return pooled ? cudaMallocFromPoolAsync(&p, b, pool, poolStream) : cudaMalloc(&p, b); }
+    cudaError_t allocate(size_t b) { return pooled ? cudaMallocFromPoolAsync(&p, b, pool->pool, pool->stream) : cudaMalloc(&p, b); }
     template <class T> void upload(const std::vector<T>& v, cudaStream_t s) {
         ensure(std::max<size_t>(1, v.size() * sizeof(T)));
         if (!v.empty()) CUDA_CHECK(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s));
@@ -266,9 +279,9 @@ struct sst_ctx {
     DevBuf commitTri[4], commitOrder, commitScratch, commitScratch4, commitScratch8;
     // The device memory of scenes that were destroyed, for the next ones: a program that prepares its
     // scene anew for every frame would otherwise pay 17 allocations and 17 device-wide frees each time.  It
-    // keeps at most kScenePoolBytes (the rest goes back when a scene is destroyed), gives that back too when
-    // an allocation fails, and goes with the context.
-    cudaMemPool_t scenePool = nullptr;
+    // keeps at most kScenePoolBytes unused (the rest goes back when a scene is destroyed or committed),
+    // gives that back too when an allocation fails, and goes with the context.
+    ScenePool scenePool;
     // wavefront buffers (store[1..] only while several waves are in flight)
     WaveStore store[kMaxWaveSets];
     DevBuf stats, film;
@@ -360,7 +373,7 @@ struct sst_scene {
     explicit sst_scene(sst_ctx* c) : ctx(c) {
         for (DevBuf* b : {&nodes, &nodes4, &nodes8, &triv, &triN, &triAux, &triVtx, &vnrm, &vuv, &mats, &texs, &texData, &ems, &envImg, &envRowCdf, &envColCdf,
                           &envHasCol, &envRowMarg, &queryJob, &record, &gTex, &gMatBase, &gMatRough, &gEmitter, &dLdI})
-            b->use(c->scenePool, c->stream);
+            b->pool = &c->scenePool;
     }
     sst_ctx* ctx;
     std::vector<HostTexture> textures;

@@ -188,7 +188,7 @@ static int outOfMemory(sst_ctx* ctx) {
     fake::budget = own + 512 * MB;
     {
         DevBuf a, b, c, d;
-        for (DevBuf* x : {&a, &b, &c}) x->use(ctx->scenePool, ctx->stream);
+        for (DevBuf* x : {&a, &b, &c}) x->pool = &ctx->scenePool;
         a.ensure(200 * MB);
         b.ensure(200 * MB);
         EXPECT(cudaStreamSynchronize(ctx->stream) == cudaSuccess);
@@ -209,6 +209,21 @@ static int outOfMemory(sst_ctx* ctx) {
         EXPECT(refused && !d.p && d.bytes == 0 && cudaGetLastError() == cudaSuccess);
     }
     return 0;
+}
+
+// What is kept of a destroyed scene does not depend on how much memory other scenes use.
+static int severalScenes(sst_ctx* ctx) {
+    const size_t MB = size_t(1) << 20;
+    sst_scene *a = makeScene(ctx), *b = makeScene(ctx);
+    EXPECT(a && b && sst_scene_commit(a, 8, 8) == SST_OK && sst_scene_commit(b, 8, 8) == SST_OK);
+    for (DevBuf* x : {&a->record, &a->gTex, &a->dLdI}) x->ensure(200 * MB);
+    b->record.ensure(100 * MB);
+    const size_t both = fake::used();
+    EXPECT(sst_scene_destroy(b) == SST_OK);
+    EXPECT(fake::used() >= both - 2 * MB && fake::used() <= both);
+    for (DevBuf* x : {&a->record, &a->gTex}) x->release();
+    EXPECT(sst_scene_commit(a, 8, 8) == SST_OK && fake::used() <= both - (500 - 256) * MB);
+    return sst_scene_destroy(a);
 }
 
 // A destroyed scene leaves at most the pool's bound behind, without another call.
@@ -254,7 +269,7 @@ static int batchFilms(sst_ctx* ctx) {
 }
 
 int main(int argc, char** argv) {
-    const std::map<std::string, int (*)(sst_ctx*)> tests = {{"query_job", queryJob}, {"overlay", overlay}, {"threads", threads}, {"failed_render", failedRender}, {"out_of_memory", outOfMemory}, {"scene_pool", scenePool}, {"batch_films", batchFilms}};
+    const std::map<std::string, int (*)(sst_ctx*)> tests = {{"query_job", queryJob}, {"overlay", overlay}, {"threads", threads}, {"failed_render", failedRender}, {"out_of_memory", outOfMemory}, {"scene_pool", scenePool}, {"several_scenes", severalScenes}, {"batch_films", batchFilms}};
     const auto it = argc > 1 ? tests.find(argv[1]) : tests.end();
     sst_ctx* ctx = nullptr;
     EXPECT(it != tests.end() && sst_create(0, &ctx) == SST_OK);

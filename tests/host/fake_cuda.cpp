@@ -40,7 +40,8 @@ void run() {
         queue.clear();
         for (auto& op : ops) op();
     }
-    for (auto p : pools) p->held = p->held < p->keep ? p->held : p->keep;  // a wait returns what is above the threshold
+    for (auto p : pools)  // a wait returns what is above the threshold, which live blocks count against too
+        if (p->live + p->held > p->keep) p->held = p->live > p->keep ? 0 : p->keep - p->live;
 }
 cudaError_t set(cudaError_t e) {
     if (e != cudaSuccess) last = e;

@@ -68,3 +68,7 @@ def test_destroyed_scenes_leave_at_most_the_bound(driver, megabytes):
 
 def test_large_batch_films_are_given_back(driver):
     run(driver, "batch_films")
+
+
+def test_what_is_kept_does_not_depend_on_other_scenes(driver):
+    run(driver, "several_scenes")
