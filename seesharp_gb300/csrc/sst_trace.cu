@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cfloat>
 #include <mutex>
 
 #include "sst_device.cuh"
@@ -72,12 +73,13 @@ struct TraceResult {
     int tri;  // leaf-ordered triangle, -1 for a miss
 };
 
-// The far bound of the wide box tests: the closest hit so far with room for the rounding of box and
-// triangle distances, and never so large that the room makes it infinite.  A child whose planes all
-// overflow to +inf (a short direction among large coordinates) then fails the test, as no triangle has
-// an infinite distance, and the entry distance of every child that passes is finite: the 4-wide node's
-// pushes tell the hit children from the others by that.
-SST_D float farBound(float t) { return fminf(t * 1.0000004f, 3.402822e38f); }
+// No ray reaches further than this (its upper end is cut to it), so that the far bound of the box tests
+// stays finite: the closest hit so far, twice enlarged for the rounding of box and triangle distances.  A
+// child whose planes all overflow to +inf (a short direction among large coordinates) then fails the
+// test, as no triangle has an infinite distance, and the entry distance of every child that passes is
+// finite: the 4-wide node's pushes tell the hit children from the others by that.
+constexpr float kFarthest = 3.40282e38f;
+static_assert(kFarthest * 1.0000004f * 1.0000004f <= FLT_MAX, "a finite far bound");
 
 struct Bvh {
     const float4* nodes;
@@ -145,7 +147,7 @@ SST_D int bestId(const float4* triv, int tri) { return tri >= 0 ? __float_as_int
 template <bool ANY, int BLOCK, int SSTACK>
 SST_D TraceResult traverse(const DevScene& scene, float3 org, float3 dir, float tmin, float tmax, int* sstack, int* errFlags) {
     const Bvh sc = bvhOf(scene);
-    TraceResult r{tmax, 0.f, 0.f, -1};
+    TraceResult r{fminf(tmax, kFarthest), 0.f, 0.f, -1};
     if (sc.nNodes == 0 || !(tmax > tmin) || originLost(org)) return r;
     int bestGid = 0x7FFFFFFF;
     RayPre pre = rayPre(dir);
@@ -245,8 +247,9 @@ SST_D float max3f(float a, float b, float c) {
     return d;
 }
 // Entry and exit distances of four child boxes from their near- and far-plane rows (x, y, z each a
-// float4 over the children; oi and of the offsets of the near and of the far planes): paired fused multiply-adds per plane row, then the three-operand
-// max / min with the ray's interval.  Bitwise the scalar fmaf / fmaxf / fminf form.
+// float4 over the children; oi and of the offsets of the near and of the far planes): paired fused
+// multiply-adds per plane row, then the three-operand max / min with the ray's interval.  Bitwise the
+// scalar fmaf / fmaxf / fminf form.
 SST_D void slab4(float4 nx, float4 fx, float4 ny, float4 fy, float4 nz, float4 fz, float3 inv, float3 oi, float3 of, float tmin, float tmax,
                  float tn[4], float tf[4]) {
     const float2 ix = make_float2(inv.x, inv.x), iy = make_float2(inv.y, inv.y), iz = make_float2(inv.z, inv.z);
@@ -278,17 +281,17 @@ SST_D void cswap(float& ka, uint32_t& ra, float& kb, uint32_t& rb) {
     ra = r;
 }
 
-// One lane's 4-wide traversal.  ncu on a million random rays of the 1M-triangle scene: L1's data stage
-// 80% busy (a node's 128-bit loads cost one pass per lane each), issue slots 57%, 8.6 of 32 lanes active;
-// DRAM 2%.  So fewer loads per node and fewer branches pay, and cheaper box arithmetic does not.  Seven
-// loads instead of eight (the child count is in the boxes: an empty child's is inside out) took
-// still-image renders of that scene from 230.6 to 222.5 ms, the straight-line pushes to 215.8 ms.
-// Measured and not kept: 256-bit loads (two passes each), 64-byte nodes with 8-bit planes (half the
+// One lane's 4-wide traversal.  ncu on the first two bounces of the 1M-triangle scene: L1's data stage 66
+// to 77% busy (a node's 128-bit loads cost one pass per lane each), issue slots 54 to 70%, 10 to 14 of 32
+// lanes active; DRAM 3 to 5%.  So fewer loads per node and fewer branches pay, and cheaper box arithmetic
+// does not.  Seven loads instead of eight (the child count is in the boxes: an empty child's is inside
+// out) took still-image renders of that scene from 230.6 to 222.5 ms, the straight-line pushes to 215.8
+// ms.  Measured and not kept: 256-bit loads (two passes each), 64-byte nodes with 8-bit planes (half the
 // passes, 20% more instructions: even), entry distances on the stack to skip nodes behind the hit (6 to
 // 15% fewer visits, but a divergent pop: 2% slower), all warps in lock step with leaves put off until
 // eight lanes have one (15 of 32 lanes active, more instructions: even).
-// It is resumable: the next node to visit, the stack depth and the closest
-// hit so far stay in the structure when trav4Run pauses.
+// It is resumable: the next node to visit, the stack depth and the closest hit so far stay in the
+// structure when trav4Run pauses.
 struct Trav4 {
     Bvh4 bvh;
     float3 org, inv, oi, of;
@@ -309,7 +312,7 @@ SST_D void trav4Begin(Trav4& s, const DevScene& sc, float3 org, float3 dir, floa
     raySlabs(sc, org, dir, s.inv, s.oi, s.of);
     s.oct = (s.inv.x < 0.0f ? 1u : 0u) | (s.inv.y < 0.0f ? 2u : 0u) | (s.inv.z < 0.0f ? 4u : 0u);
     s.tmin = tmin;
-    s.r = TraceResult{tmax, 0.f, 0.f, -1};
+    s.r = TraceResult{fminf(tmax, kFarthest), 0.f, 0.f, -1};
     s.sp = 0;
     s.ref = 0;  // root
     s.done = bvh.nNodes4 == 0 || !(tmax > tmin) || originLost(org) || noShear(s.pre);
@@ -340,7 +343,7 @@ SST_D bool trav4Run(Trav4& s, int* sstack, int* lstack, int* errFlags, int pause
             const float4 nx = __ldg(nd + ox), fx = __ldg(nd + 1 - ox), ny = __ldg(nd + 2 + oy), fy = __ldg(nd + 3 - oy);
             const float4 nz = __ldg(nd + 4 + oz), fz = __ldg(nd + 5 - oz);
             const float4 rf = __ldg(nd + 6);
-            const float hitT = farBound(s.r.t);
+            const float hitT = s.r.t * 1.0000004f;  // conservative far bound (box/triangle rounding)
             float key[4];
             uint32_t cr[4];
             const float* RF = &rf.x;
@@ -441,7 +444,7 @@ SST_D uint32_t visit8(const Trav8& s, uint32_t node) {
     const float4* nd = s.bvh.nodes8 + 15 * (size_t)node;
     const int ox = (int)(s.oct & 1u), oy = (int)((s.oct >> 1) & 1u), oz = (int)((s.oct >> 2) & 1u);
     const uint32_t valid = __float_as_uint(__ldg(&nd[14].x)) & 0xFFu;
-    const float hitT = farBound(s.r.t);
+    const float hitT = s.r.t * 1.0000004f;  // conservative far bound (box/triangle rounding)
     uint32_t hm = 0;
     // two halves of four children (24 box floats live at a time); near planes: lo for a positive
     // direction component, hi for a negative one
@@ -471,7 +474,7 @@ SST_D void trav8Begin(Trav8& s, const DevScene& sc, float3 org, float3 dir, floa
     raySlabs(sc, org, dir, s.inv, s.oi, s.of);
     s.oct = (s.inv.x < 0.0f ? 1u : 0u) | (s.inv.y < 0.0f ? 2u : 0u) | (s.inv.z < 0.0f ? 4u : 0u);
     s.tmin = tmin;
-    s.r = TraceResult{tmax, 0.f, 0.f, -1};
+    s.r = TraceResult{fminf(tmax, kFarthest), 0.f, 0.f, -1};
     s.sp = 0;
     s.node = 0;
     s.done = bvh.nNodes8 == 0 || !(tmax > tmin) || originLost(org) || noShear(s.pre);
