@@ -229,7 +229,8 @@ int sst_autotune(sst_scene* scene, const SstPathTracerParams* params, int32_t tr
 /* ---- allocation-free occlusion query: no counterpart in the reference --------------------------
  * The same any-hit queries as sst_occluded, with the same arguments and the same results, but the
  * call allocates no memory: no cudaMalloc or cudaFree, and no allocating CUDA library routine.
- * sst_occluded allocates its temporary device buffers on every call.  Some callers cannot do that:
+ * sst_occluded grows its context's buffers whenever a query is larger than any before it, which frees
+ * and allocates device memory.  Some callers cannot have that:
  *  - a caller whose device memory is fully budgeted, e.g. one that shares the GPU with another
  *    process holding the rest of it, where a new allocation can fail in the middle of a frame;
  *  - a caller on a latency-bound loop (shadow or picking queries per frame): cudaFree waits for

@@ -32,10 +32,11 @@ namespace {
 constexpr float kCt = 0.25f;
 constexpr float kCi = 1.0f;
 // PLOC rounds between two looks at the cluster count.  A round leaves 70 to 80% of the clusters, so the
-// third one's grid is at most twice what it needs.  With a look (four read-backs and a wait) after every
-// one of the 61 rounds of 614K triangles the GPU idled for half of a commit: 8.8 ms against 5.1 ms with a
-// look after every third round and one block for the last half of them (and the wide tree's levels
-// launched from bounds); 36 triangles: 1.11 against 0.27 ms.
+// third one's grid is at most twice what it needs.  Commits of 10K / 102K / 614K / 1M / 2M triangles with a
+// look after every round: 1.11 / 2.35 / 4.68 / 6.49 / 11.17 ms, every second: 1.09 / 2.20 / 4.51 / 6.29 / 10.94,
+// every third: 1.07 / 2.17 / 4.48 / 6.25 / 10.88, every fourth: 1.07 / 2.16 / 4.44 / 6.18 / 10.84, every sixth:
+// 1.08 / 2.16 / 4.39 / 6.14 / 10.80.  (With four read-backs and a wait after each of the 61 rounds, no block
+// that does the last half of them and a read-back per level of the wide tree: 614K triangles 8.8 ms.)
 constexpr int kPlocRounds = 3;
 
 __device__ __forceinline__ int floatOrd(float f) {

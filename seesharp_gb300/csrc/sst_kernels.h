@@ -40,13 +40,13 @@ void launch_trace_shadow(const TraceTuning& t, const DevJob* jobs, const uint32_
 // n rays as interleaved records (origin and tmin, direction and tmax), 16-byte aligned.
 void launch_trace_query(const TraceTuning& t, const DevJob* jobs, const float4* rays, int n, int* work, float4* hits, int* occl, DevStats* stats,
                         bool anyHit, cudaStream_t s);
+void launch_wave_advance(int* wave, int by, cudaStream_t s);
+// Writes the shade order of a bounce's queue (surface hits first) into order[0, *nIn).
+void launch_partition(bool replay, const uint32_t* depth, const float4* hits, const int* nIn, int* order, int* counts, int maxItems, cudaStream_t s);
 // shadeBlocks: the resident blocks per SM of the forward variant with GenericMaterials: the
 // default build (8, 64 registers) or a denser one (10, 12 or 14: 48, 40 or 32 registers, more warps,
 // more spilling); one shadow ray per technique has every build, more shadow rays the default one.
 // The denser builds live in sst_shade_occ.cu.
-void launch_wave_advance(int* wave, int by, cudaStream_t s);
-// Writes the shade order of a bounce's queue (surface hits first) into order[0, *nIn).
-void launch_partition(bool replay, const uint32_t* depth, const float4* hits, const int* nIn, int* order, int* counts, int maxItems, cudaStream_t s);
 bool shadeBlocksValid(int blocks);
 // The split form (sst_shade_split.cu), forward, GenericMaterials, one shadow ray per technique: two
 // kernels per bounce, A.rec must hold kShadeRec * cap float4.  blocks: 14 selects the dense build of

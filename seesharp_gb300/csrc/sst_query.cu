@@ -13,17 +13,17 @@ void uploadQueryJob(sst_scene* s) {
 }
 
 // Queries of up to this many rays between host arrays go through page-locked memory that the kernels
-// read and write in place, instead of two copies.  Closest hits of 97 / 1024 / 2048 / 4096 rays on the
-// Cornell box: 38 / 48 / 51 / 60 us with copies, 33 / 40 / 47 / 63 us in place (its 48-byte records
-// make the link the bound from there on); occlusion of 97 / 4096 / 8192 / 16384 rays: 32 / 43 / 44 / 46
-// against 25 / 33 / 38 / 51 us.  (65 to 101 us before, with the rays split by two strided copies and the
-// job table, the counters and the statistics uploaded and read back each time.)
+// read and write in place, instead of two copies.  In us, in place / copied, on the Cornell box, 205K and 1M
+// triangles: closest hits of 97 rays 33 / 38, 48 / 53, 72 / 84, of 2048 rays 43 / 52, 67 / 76, 95 / 102, of 4096
+// 52 / 53, 82 / 85, 114 / 122, of 8192 71 / 59, 109 / 102, 137 / 127 (the 48-byte records make the link the
+// bound); occlusion of 97 rays 26 / 34, 37 / 45, 54 / 60, of 8192 37 / 44, 74 / 80, 93 / 104, of 16384 50 / 46,
+// 78 / 82, 117 / 119, of 32768 87 / 51, 128 / 99, 143 / 111.  The lines lie where every scene gains.
 constexpr int kTraceInPlace = 2048, kOcclInPlace = 8192;
 
 // Trace / IsOccluded over n rays.  The traversal reads the SstRay records where they are (device
-// arrays on a 16-byte boundary, apart from the results) or from one copy of them; sst_trace's SstHit records are expanded on the
-// device from the traversal's (t, u, v, triangle) records.  The buffers are the context's and only
-// grow, so repeated queries of the same size allocate nothing.
+// arrays on a 16-byte boundary, apart from the results) or from one copy of them; sst_trace's SstHit
+// records are expanded on the device from the traversal's (t, u, v, triangle) records.  The buffers are
+// the context's and only grow, so repeated queries of the same size allocate nothing.
 static void runQuery(sst_scene* s, const SstRay* rays, int n, SstHit* hits, int32_t* occl, int memory, bool anyHit) {
     static_assert(sizeof(SstHit) == sizeof(SstHitDev), "hit layout");
     static_assert(sizeof(SstRay) == 2 * sizeof(float4), "ray layout");

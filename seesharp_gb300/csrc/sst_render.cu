@@ -1,8 +1,9 @@
 // PathTracerBase.Render (Integrators/PathTracer.cs:199-267) as the wavefront renderer: the
 // (job, iteration, pixel) paths are cut into waves that fit the path-state buffers; each wave runs
-// camera -> {closest hit, shade, shadow rays} x depth -> film fold on the context's stream, replayed
-// as one CUDA graph per wave.  Also the launch tuning and autotuner, the frame-buffer layers and
-// batched rendering.
+// camera -> {closest hit, shade, shadow rays} x depth -> film fold.  Up to three waves are in flight, each
+// on its own buffers and streams with the folds in wave order on the context's; renders of many waves
+// replay a captured CUDA graph per wave, shorter ones launch the kernels directly.  Also the launch
+// tuning and autotuner, the frame-buffer layers and batched rendering.
 #include "sst_host.h"
 
 // ---------------------------------------------------------------------------------------------
@@ -124,11 +125,18 @@ static void planWaves(std::vector<JobIn>& jobs, int cap, bool iterationPerWave, 
 
 // Waves of up to this many paths are shaded in queue order: they leave most of the GPU idle, so the shade
 // launch lasts as long as its slowest warp in either order, and the order is one more launch per bounce.
-// With the order and without it: Cornell box of 160 x 90, 1 sample, 370 and 346 us, of 256 x 192 439 and
-// 412, sphere field of 256 x 192 858 and 849; above the line the sphere field loses (512 x 512: 1423 and
-// 1446).  The replay keeps the order at every size (its sums depend on it, k_partition_warp).
+// Time in queue order over that in order, one wave of 64^2 to 256^2 paths, depths 5 and 10, one and two shadow rays:
+// Cornell box 0.87 to 0.91, environment-lit box 0.90 to 0.93, textured box 0.89 to 0.94, sphere field of 31K
+// triangles 0.94 to 0.96, of 1M triangles 0.96 to 1.01; above the line the field loses (60 spheres, 512 x 512: 1446
+// us in queue order, 1423 in order).  The replay keeps the order at every size (its sums depend on it, k_partition_warp).
 constexpr int kOrderItems = 1 << 16;
-constexpr size_t kGraphWaves = 8;  // waves from which several sets of a forward pass replay captured graphs
+// Waves from which a forward pass on several sets replays captured graphs.  Capturing, instantiating and
+// destroying the graphs takes 0.2 (depth 5) to 1 ms (depth 32) in which the GPU has nothing to do; launching
+// a wave kernel by kernel takes the host longer than replaying it.  Time of direct launches over that of graphs, Cornell
+// box and 205K-triangle sphere field, waves of 2^14 to 2^20 paths, depths 5, 16 and 32: 2 waves 0.59 to 0.91,
+// 3 waves 0.67 to 0.95, 5 waves 0.80 to 0.97, 8 waves 0.94 to 1.02, 16 waves 0.99 to 1.13, 32 waves 0.99 to 1.23
+// (the gain of graphs is largest for small and deep waves).
+constexpr size_t kGraphWaves = 8;
 
 // Renders the jobs' iterations [iterFirst, iterEnd) into their device films.
 // paths: instead of the jobs' iteration ranges, render exactly these single-path chunks (one
@@ -218,7 +226,7 @@ void renderJobs(sst_ctx* c, std::vector<JobIn>& jobs, SstRenderStats* out, bool 
     // Several waves in flight: consecutive waves take turns over nSets buffer sets and their
     // streams, so that one wave's last bounces (few paths, latency-bound) run beside the next
     // wave's first ones; the film folds run in wave order on the context's stream.  Not for the
-    // technique pyramid (single-set buffers) and without graphs.
+    // technique pyramid (single-set buffers), kernel timing, time limits, depths above 32 and SST_GRAPH=0.
     // SST_WAVES_IN_FLIGHT: 1 to kMaxWaveSets (default 2).
     const char* wf = getenv("SST_WAVES_IN_FLIGHT");
     const int wantSets = std::min(kMaxWaveSets, std::max(1, wf ? atoi(wf) : 2));
@@ -411,10 +419,7 @@ void renderJobs(sst_ctx* c, std::vector<JobIn>& jobs, SstRenderStats* out, bool 
         // The bounces of a wave and the advance of its set's wave index run on the set's stream; the
         // folds are plain launches on the context's stream, in wave order, each after its wave's bounces
         // (evDone) and before the set's next wave reuses the estimates (evFolded).  From kGraphWaves waves
-        // on a set's wave is captured once and replayed.  Capturing, instantiating and destroying the
-        // graphs takes about 0.5 ms in which the GPU has nothing to do, launching a wave kernel by kernel
-        // about 0.1 ms beside a running one: 4 waves (509 x 383, 32 samples) 7.93 ms with graphs, 7.73
-        // without; 5 waves (40 small jobs) 7.57 against 7.38 ms; 32 waves the same either way.  The replay
+        // on a set's wave is captured once and replayed (see there).  The replay
         // keeps the graphs: launched one by one its waves meet differently, and the 32-bit gradient sums round
         // by the order of their additions (512 x 512, 32 samples, radiance gradients against
         // the mean of 8 runs with graphs: those 1e-5 apart, without 3e-5, and 3e-4 in one run of eight).

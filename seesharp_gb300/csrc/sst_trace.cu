@@ -282,7 +282,7 @@ SST_D void cswap(float& ka, uint32_t& ra, float& kb, uint32_t& rb) {
 }
 
 // One lane's 4-wide traversal.  ncu on the first two bounces of the 1M-triangle scene: L1's data stage 66
-// to 77% busy (a node's 128-bit loads cost one pass per lane each), issue slots 54 to 70%, 10 to 14 of 32
+// to 78% busy (a node's 128-bit loads cost one pass per lane each), issue slots 54 to 70%, 10 to 14 of 32
 // lanes active; DRAM 3 to 5%.  So fewer loads per node and fewer branches pay, and cheaper box arithmetic
 // does not.  Seven loads instead of eight (the child count is in the boxes: an empty child's is inside
 // out) took still-image renders of that scene from 230.6 to 222.5 ms, the straight-line pushes to 215.8
